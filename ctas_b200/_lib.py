@@ -23,6 +23,7 @@ FLAG_NO_WRITEBACK = 0x1
 FLAG_SHIPPED_INDEX = 0x2
 FLAG_CHECKED = 0x100
 FLAG_TEST_TIMEOUT = 0x200
+FLAG_GROUPS = 0x400
 
 
 class Opts(C.Structure):

@@ -25,6 +25,8 @@ int bp_fast_search(const std::function<float(int)> &time_ms, bool all_variants);
 // (device, W, N, store, interp) -- the first launch of a shape runs
 // bp_fast_search on one slice of that launch (synchronising the stream).
 int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested);
+// True when CTAS_FBP_TILE names a tile.
+bool bp_fast_tile_forced();
 cudaError_t launch_bp_fast(const BpLaunch &a, cudaStream_t st, int tile);
 // Same kernel with every shared-memory gather checked against its window
 // (violations set bit 8 of *a.err and read 0); for tests.

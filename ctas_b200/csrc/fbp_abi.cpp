@@ -30,6 +30,7 @@
 #include "../../include/ctas_fbp.h"
 #include "../../include/ctas_volume.h"
 #include "bp_fast.hpp"
+#include "bp_quad.hpp"
 #include "fbp_host.hpp"
 #include "fbp_kernels.hpp"
 
@@ -121,6 +122,8 @@ struct Consts {
 // One set of work buffers (the host stack call double-buffers two sets).
 struct WorkSet {
   DevBuf raw, filt, scale, slice, part, minmax, ring_avg, ring;
+  DevBuf quad;     // interleaved rows of the four-slice groups, with their slack
+  DevBuf dense;    // dense filtered rows to be written back (four-slice groups)
   DevBuf samples;  // converted output samples of the volume call
   int64_t slices = 0;
   cudaEvent_t ev_in = nullptr, ev_done = nullptr, ev_out = nullptr;
@@ -152,7 +155,7 @@ struct ctas_fbp {
   // them too; off = column of sample 0
   bool wide = false;
   int64_t off = ctas::kRowOff;
-  int device = 0;
+  int device = 0, sms = 148;
   std::shared_ptr<Consts> dc;
   cudaStream_t stream = nullptr, s_in = nullptr, s_out = nullptr;
   WorkSet ws[2];
@@ -195,6 +198,8 @@ struct ctas_fbp {
       w.ring_avg.release();
       w.ring.release();
       w.samples.release();
+      w.quad.release();
+      w.dense.release();
     }
     for (auto *r : {vin, vout})
       for (int i = 0; i < 3; i++) {
@@ -234,12 +239,50 @@ void init_streams(ctas_fbp *h) {
   *h->err_host = 0;
 }
 
-// Sizes one work set for S slices.  The padded filtered buffer is zeroed on
-// allocation: its pad columns are never written afterwards.
+// Whether stacks of this handle may go through the four-slice kernel: float32
+// rows, the reference's truncation on rows that serve it without branches
+// (sines >= 0, or the wide layout), and no tile asked for by id.
+bool quad_capable(const ctas_fbp *h) {
+  return h->store == CTAS_STORE_F32 && h->interp == CTAS_INTERP_TRUNC &&
+         (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
+         !ctas::bp_fast_tile_forced();
+}
+
+// How many of S slices (the first ones) go through the four-slice kernel: whole
+// groups, and a group of the last three.  One or two slices left over take the
+// one-slice kernel: a group's time is that of 2.2 slices of 1800 x 2560 alone.
+int64_t quad_count(const ctas_fbp *h, int64_t S) {
+  if (S < 3 || !quad_capable(h)) return 0;
+  const int64_t rest = S % ctas::kQuadSlices, n = rest == 3 ? S : S - rest;
+  if (!(h->flags & CTAS_FLAG_GROUPS) && !ctas::bp_quad_pays(h->out_rows, h->out_cols, n, h->sms))
+    return 0;
+  return n;
+}
+
+int64_t quad_groups(int64_t slices) { return (slices + ctas::kQuadSlices - 1) / ctas::kQuadSlices; }
+
+// First row of the interleaved buffer.
+float *quad_rows(const WorkSet &w) {
+  return w.quad.as<float>() + ctas::kQuadSlices * ctas::kQuadSlack;
+}
+
+// Sizes one work set for S slices or fewer.  The padded filtered buffers are zeroed
+// on allocation: their pad columns are never written afterwards.
 void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw) {
   const int64_t N = h->N, W = h->W;
   if (need_raw) w.raw.ensure(sizeof(float) * (size_t)(S * N * W));
-  if (w.filt.ensure(elem_bytes(h->store) * (size_t)(S * N * h->Wp)))
+  const int64_t n4 = quad_count(h, S);
+  // most slices that a launch of at most S leaves to the one-slice kernel: those below
+  // the first count that forms groups, or a rest of two
+  int64_t alone = S;
+  if (n4 > 0)
+    for (alone = 2; quad_count(h, alone + 1) == 0;) alone++;
+  if (n4 > 0) {
+    const int64_t words = quad_groups(S) * N * h->Wp + 2 * ctas::kQuadSlack;
+    if (w.quad.ensure(sizeof(float) * ctas::kQuadSlices * (size_t)words))
+      cuda_check(cudaMemset(w.quad.p, 0, w.quad.bytes), "cudaMemset");
+  }
+  if (w.filt.ensure(elem_bytes(h->store) * (size_t)(alone * N * h->Wp)))
     cuda_check(cudaMemset(w.filt.p, 0, w.filt.bytes), "cudaMemset");
   if (h->store != 0) w.scale.ensure(sizeof(float) * (size_t)(S * N));
   w.slice.ensure(sizeof(float) * (size_t)(S * h->out_rows * h->out_cols));
@@ -303,8 +346,10 @@ const float *run_ring(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaSt
   return w.ring.as<float>();
 }
 
-// Filter S slices of x (device, dense S x N x W) into w.filt.
-void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t st) {
+// Filter S slices of x (device, dense S x N x W): the first quad_count() into w.quad,
+// the others into w.filt; densely into `dense` too, unless null (float32 store).
+void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t st,
+                float *dense = nullptr) {
   const float *ring = run_ring(h, x, S, w, st);
   if (h->contrast == CTAS_ABS) {
     cuda_check(ctas::launch_minmax(x, h->N * h->W, h->N * h->W, (int)S, w.part.as<float2>(),
@@ -334,16 +379,40 @@ void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t
   a.guard = h->interp == CTAS_INTERP_TRUNC ? 1 : 0;
   a.ring = ring;
   a.off = (int)h->off;
+  a.dense = dense;
+  const int64_t n4 = quad_count(h, S), rest = S - n4;
   KernelTimer tm(h, CTAS_KERNEL_FILTER, st);
-  cuda_check(ctas::launch_filter(a, st), "filter kernel");
-  if (h->wide) {
-    cuda_check(ctas::launch_halo(w.filt.as<float>(), h->N * h->Wp, (int)h->N, (int)h->W,
-                                 (int)h->Wp, (int)h->off, (int)S, st),
-               "halo kernel");
+  if (n4 > 0) {
+    ctas::FilterLaunch b = a;
+    b.quad = 1;
+    b.q = quad_rows(w);
+    b.q_slice_stride = ctas::kQuadSlices * h->N * h->Wp;
+    b.S = (int)n4;
+    cuda_check(ctas::launch_filter(b, st), "filter kernel");
     h->launches += 1;
+    if (h->wide) {
+      cuda_check(ctas::launch_halo_quad(quad_rows(w), h->N * h->Wp, (int)h->N, (int)h->W,
+                                        (int)h->Wp, (int)h->off, (int)n4, st),
+                 "halo kernel");
+      h->launches += 1;
+    }
+    a.x += n4 * h->N * h->W;
+    if (a.minmax) a.minmax += n4;
+    if (a.ring) a.ring += n4 * h->W;
+    if (a.dense) a.dense += n4 * h->N * h->W;
+    a.S = (int)rest;
+  }
+  if (rest > 0) {
+    cuda_check(ctas::launch_filter(a, st), "filter kernel");
+    h->launches += 1;
+    if (h->wide) {
+      cuda_check(ctas::launch_halo(w.filt.as<float>(), h->N * h->Wp, (int)h->N, (int)h->W,
+                                   (int)h->Wp, (int)h->off, (int)rest, st),
+                 "halo kernel");
+      h->launches += 1;
+    }
   }
   tm.done();
-  h->launches += 1;
 }
 
 // centers_dev: per-slice centres (device) of S slices that all backproject
@@ -380,6 +449,23 @@ void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, 
   b.err = h->err.as<int>();
   b.interp = h->interp;
   b.lin = h->interp == CTAS_INTERP_LINEAR ? h->dc->lin.as<double2>() : nullptr;
+  const int64_t n4 = centers_dev ? 0 : quad_count(h, S);
+  if (n4 > 0) {
+    KernelTimer tm(h, CTAS_KERNEL_BACKPROJECT, st);
+    ctas::BpLaunch g = b;
+    g.q = quad_rows(w);
+    g.S = (int)n4;
+    const cudaError_t e = ctas::launch_bp_quad(g, st, (h->flags & CTAS_FLAG_CHECKED) != 0);
+    if (e != cudaSuccess)
+      cuda_check(e, (std::string("backprojection kernel: ") + ctas::bp_quad_error_detail()).c_str());
+    tm.done();
+    h->launches += 1;
+    h->last_kernel = 2;
+    h->last_tile = -1;
+    if (n4 == S) return;
+    b.S = (int)(S - n4);
+    b.out = out + n4 * b.out_slice_stride;
+  }
   const bool fast = ctas::bp_fast_supported(b) &&
                     (h->interp == CTAS_INTERP_LINEAR || h->sines_nonneg || h->wide);
   int tile = -1;
@@ -474,12 +560,18 @@ ctas_fbp *checked(ctas_fbp *h) {
   return h;
 }
 
+// Chunks of whole groups where stacks go through the four-slice kernel.
+int64_t whole_groups(const ctas_fbp *h, int64_t S, int64_t C) {
+  if (quad_count(h, S) == 0) return C;
+  return std::min<int64_t>(S, quad_groups(C) * ctas::kQuadSlices);
+}
+
 int64_t device_chunk(const ctas_fbp *h, int64_t S) {
   if (h->chunk > 0) return std::min<int64_t>(h->chunk, S);
   const double per = (double)h->N * h->Wp * elem_bytes(h->store) + 8.0 * h->N;
   int64_t cmax = std::max<int64_t>(1, (int64_t)(4.0e9 / per));
   const int64_t nch = (S + cmax - 1) / cmax;
-  return (S + nch - 1) / nch;
+  return whole_groups(h, S, (S + nch - 1) / nch);
 }
 
 int64_t host_chunk(const ctas_fbp *h, int64_t S) {
@@ -490,22 +582,27 @@ int64_t host_chunk(const ctas_fbp *h, int64_t S) {
   // keep at least a few chunks so copies overlap compute
   cmax = std::min<int64_t>(cmax, std::max<int64_t>(1, (S + 3) / 4));
   const int64_t nch = (S + cmax - 1) / cmax;
-  return (S + nch - 1) / nch;
+  return whole_groups(h, S, (S + nch - 1) / nch);
 }
 
 // Chunk sizes of the host stack call: chunks of C slices, entered and left
 // through chunks of 2, 4, 8, ... slices, so that the first upload and the last
-// download (the copies no compute overlaps) are short.
-std::vector<int64_t> chunk_plan(int64_t n, int64_t C) {
+// download (the copies no compute overlaps) are short.  unit: chunks but the last of the
+// middle ones are multiples of it (C is one, or n).
+std::vector<int64_t> chunk_plan(int64_t n, int64_t C, int64_t unit) {
   std::vector<int64_t> up;
   int64_t ramp = 0;
-  for (int64_t c = 2; c < C && ramp + 2 * c <= n / 2; c *= 2) {
+  for (int64_t c = std::max<int64_t>(2, unit); c < C && ramp + 2 * c <= n / 2; c *= 2) {
     up.push_back(c);
     ramp += 2 * c;
   }
   std::vector<int64_t> plan(up.begin(), up.end());
   const int64_t mid = n - ramp, nmid = (mid + C - 1) / C;
-  for (int64_t i = 0; i < nmid; i++) plan.push_back(mid * (i + 1) / nmid - mid * i / nmid);
+  auto edge = [&](int64_t i) {
+    return std::min(mid, (mid * i / nmid + unit - 1) / unit * unit);
+  };
+  for (int64_t i = 0; i < nmid; i++)
+    if (edge(i + 1) > edge(i)) plan.push_back(edge(i + 1) - edge(i));
   plan.insert(plan.end(), up.rbegin(), up.rend());
   return plan;
 }
@@ -732,6 +829,8 @@ int ctas_fbp_create(ctas_fbp **out, int64_t n_angles, int64_t width, int32_t con
     else h->device = o.device;
     if (h->device >= ndev) ctas::fail(CTAS_E_ARG, "device ordinal out of range");
     DeviceGuard g(h->device);
+    cuda_check(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device),
+               "cudaDeviceGetAttribute");
 
     // constants: twiddles, window in the FFT's output order (divided by P),
     // angle table
@@ -809,6 +908,7 @@ int ctas_fbp_clone(const ctas_fbp *src, ctas_fbp **out) {
     h->wide = src->wide;
     h->off = src->off;
     h->device = src->device;
+    h->sms = src->sms;
     h->dc = src->dc;
     init_streams(h.get());
     *out = h.release();
@@ -1040,7 +1140,13 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     const int64_t C = host_chunk(h, n_slices);
     const bool wb = !(h->flags & CTAS_FLAG_NO_WRITEBACK);
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
-    for (auto &w : h->ws) ensure_set(h, w, C, true);
+    // four-slice groups are filtered into interleaved rows: the rows to write back are
+    // stored densely beside them
+    const bool dense = wb && quad_count(h, C) > 0;
+    for (auto &w : h->ws) {
+      ensure_set(h, w, C, true);
+      if (dense) w.dense.ensure(sizeof(float) * (size_t)(C * NW));
+    }
     // If a later chunk fails, copies of earlier chunks into the caller's host
     // buffers may still be queued: drain all three streams before returning,
     // so the caller may free those buffers once the call has returned.
@@ -1068,7 +1174,8 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     }
     // three-stream pipeline: host->device (s_in), compute (stream),
     // device->host (s_out); two work sets alternate.
-    const std::vector<int64_t> plan = chunk_plan(n_slices, C);
+    const bool groups = h->chunk <= 0 && quad_count(h, n_slices) > 0;
+    const std::vector<int64_t> plan = chunk_plan(n_slices, C, groups ? ctas::kQuadSlices : 1);
     int64_t k = 0, s0 = 0;
     for (const int64_t S : plan) {
       WorkSet &w = h->ws[k & 1];
@@ -1078,7 +1185,7 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
                  "cudaMemcpyAsync");
       cuda_check(cudaEventRecord(w.ev_in, h->s_in), "cudaEventRecord");
       cuda_check(cudaStreamWaitEvent(h->stream, w.ev_in, 0), "cudaStreamWaitEvent");
-      run_filter(h, w.raw.as<float>(), S, w, h->stream);
+      run_filter(h, w.raw.as<float>(), S, w, h->stream, dense ? w.dense.as<float>() : nullptr);
       run_bp(h, w, S, center, w.slice.as<float>(), h->stream);
       // 16-bit stores: the written-back rows are the stored samples times
       // their row scales, formed by the unpad kernel in w.raw
@@ -1094,7 +1201,11 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
       cuda_check(cudaMemcpyAsync(slices + s0 * OO, w.slice.p, sizeof(float) * (size_t)(S * OO),
                                  cudaMemcpyDeviceToHost, h->s_out),
                  "cudaMemcpyAsync");
-      if (wb && h->store == 0) {
+      if (dense) {
+        cuda_check(cudaMemcpyAsync(sinos + s0 * NW, w.dense.p, sizeof(float) * (size_t)(S * NW),
+                                   cudaMemcpyDeviceToHost, h->s_out),
+                   "cudaMemcpyAsync");
+      } else if (wb && h->store == 0) {
         // float32 store: the filtered rows sit in w.filt, W samples from column
         // off of every Wp-sample row (slices follow at N rows each), and one
         // pitched copy brings them back

@@ -31,6 +31,16 @@ inline int64_t padded_pitch(int64_t W) { return ((W + kRowOff + 1 + 7) / 8) * 8 
 inline int64_t wide_offset(int64_t W) { return ((W + 16 + 7) / 8) * 8; }
 inline int64_t wide_pitch(int64_t W) { return wide_offset(W) + ((2 * W + 16 + 7) / 8) * 8; }
 
+// Interleaved layout, for stacks of slices that share one geometry: sample k of row r
+// of slice s is lane s % 4 of the 16-byte word at
+//   ((s / 4) * N + r) * Wp + off + k
+// (either column layout above, guard and halo columns included), so that the four
+// slices of a group are read by one load.  kQuadSlack words are allocated before
+// the first row and behind the last: windows of tiles at the rim of the disc reach
+// past the rows.
+constexpr int kQuadSlices = 4;
+constexpr int kQuadSlack = 256;
+
 struct FilterLaunch {
   const float *x;            // S x N x W input rows
   int64_t x_slice_stride;    // elements between slices of x
@@ -54,6 +64,10 @@ struct FilterLaunch {
                              // with a window symmetric about 0 this is the row's
                              // circular convolution of length W (unpadded filter)
   int off;                   // column of sample 0 in the output rows; 0 = kRowOff
+  int quad;                  // 1: interleaved layout (float32; q_slice_stride is then a
+                             // group's, in floats)
+  float *dense;              // also store the filtered rows densely, S x N x W (float32;
+                             // not with a reduced-precision store), or null
 };
 cudaError_t launch_filter(const FilterLaunch &a, cudaStream_t st);
 // Uneven batch (float32 store, filtering contrasts): jobs_dev[k] describes
@@ -94,6 +108,9 @@ cudaError_t launch_unpad(const void *q, int64_t q_slice_stride, const float *row
 // from the filtered samples of the neighbouring rows of each slice.
 cudaError_t launch_halo(float *q, int64_t q_slice_stride, int N, int W, int Wp, int off, int S,
                         cudaStream_t st);
+// The same for S slices in the interleaved layout (q_group_stride in words).
+cudaError_t launch_halo_quad(float *q, int64_t q_group_stride, int N, int W, int Wp, int off, int S,
+                             cudaStream_t st);
 
 struct BpLaunch {
   const void *q;             // padded filtered rows (see above)

@@ -331,9 +331,14 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
   // rows go straight from the last inverse stage to global memory unless a
   // row-wide epilogue (REF running sum, reduced-precision scale) needs them
   const bool direct = ns >= 2 && a.contrast != 1 && a.store == 0;
-  T *q0 = reinterpret_cast<T *>(a.q) + sl * a.q_slice_stride + (int64_t)r0 * a.Wp +
-          (a.off ? a.off : kRowOff);
-  T *q1 = q0 + a.Wp;
+  // es: elements between samples of a row, ep: between rows
+  const int es = a.quad ? kQuadSlices : 1;
+  const int64_t ep = (int64_t)es * a.Wp;
+  T *q0 = reinterpret_cast<T *>(a.q) + (a.quad ? (sl / kQuadSlices) * a.q_slice_stride + sl % kQuadSlices
+                                               : sl * a.q_slice_stride) +
+          (int64_t)r0 * ep + (a.off ? a.off : kRowOff) * es;
+  T *q1 = q0 + ep;
+  float *d0 = a.dense ? a.dense + ((int64_t)sl * N + r0) * W : nullptr;
 
   if (ns >= 2) {
     const int R = a.radix[0];
@@ -363,19 +368,23 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
     auto store = [&](int p, float2 z) {
       const int c = p - zs;
       if (c < 0 || c >= W) return;
-      q0[c] = to_store<T>(z.x);
-      if (has1) q1[c] = to_store<T>(z.y);
+      q0[c * es] = to_store<T>(z.x);
+      if (has1) q1[c * es] = to_store<T>(z.y);
+      if (d0) {
+        d0[c] = z.x;
+        if (has1) d0[W + c] = z.y;
+      }
       if (c == 0 && a.guard) {
         // column -1 repeats sample 0; column W of the previous row is sample 0
         // of this row (flat-buffer read one past the row end)
-        q0[-1] = to_store<T>(z.x);
-        if (r0 > 0) q0[W - a.Wp] = to_store<T>(z.x);
+        q0[-es] = to_store<T>(z.x);
+        if (r0 > 0) q0[W * es - ep] = to_store<T>(z.x);
         if (has1) {
-          q1[-1] = to_store<T>(z.y);
-          q0[W] = to_store<T>(z.y);
-          if (r1 == N - 1) q1[W] = to_store<T>(0.f);
+          q1[-es] = to_store<T>(z.y);
+          q0[W * es] = to_store<T>(z.y);
+          if (r1 == N - 1) q1[W * es] = to_store<T>(0.f);
         } else {
-          q0[W] = to_store<T>(0.f);
+          q0[W * es] = to_store<T>(0.f);
         }
       }
     };
@@ -448,22 +457,26 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
 
   for (int c = threadIdx.x; c < W; c += blockDim.x) {
     const float2 z = sm[sidx(zs + c)];
-    q0[c] = to_store<T>(z.x * i0);
-    if (has1) q1[c] = to_store<T>(z.y * i1);
+    q0[c * es] = to_store<T>(z.x * i0);
+    if (has1) q1[c * es] = to_store<T>(z.y * i1);
+    if (d0) {
+      d0[c] = z.x;
+      if (has1) d0[W + c] = z.y;
+    }
   }
   if (threadIdx.x == 0 && a.guard) {
     const float2 z = sm[sidx(zs)];
     // column -1 repeats sample 0; column W of the previous row is sample 0 of
     // this row (flat-buffer read one past the row end)
-    q0[-1] = to_store<T>(z.x * i0);
+    q0[-es] = to_store<T>(z.x * i0);
     if (a.store == 0) {
-      if (r0 > 0) q0[W - a.Wp] = to_store<T>(z.x);
+      if (r0 > 0) q0[W * es - ep] = to_store<T>(z.x);
       if (has1) {
-        q1[-1] = to_store<T>(z.y * i1);
-        q0[W] = to_store<T>(z.y);
-        if (r1 == N - 1) q1[W] = to_store<T>(0.f);
+        q1[-es] = to_store<T>(z.y * i1);
+        q0[W * es] = to_store<T>(z.y);
+        if (r1 == N - 1) q1[W * es] = to_store<T>(0.f);
       } else {
-        q0[W] = to_store<T>(0.f);
+        q0[W * es] = to_store<T>(0.f);
       }
     } else {
       // reduced precision: each row is scaled separately, so the one-past-
@@ -480,6 +493,13 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
 template <typename T>
 __global__ void __launch_bounds__(kFftThreads) filter_rows_kernel(FilterLaunch a) {
   filter_pair<T>(a, blockIdx.x, blockIdx.y);
+}
+
+// Interleaved layout: the four slices of a group write the same 32-byte sectors, so
+// their blocks for one row pair are neighbours and the sectors fill in L2.
+__global__ void __launch_bounds__(kFftThreads) filter_quad_kernel(FilterLaunch a) {
+  const int sl = kQuadSlices * blockIdx.y + (blockIdx.x & (kQuadSlices - 1));
+  if (sl < a.S) filter_pair<float>(a, blockIdx.x / kQuadSlices, sl);
 }
 
 // Uneven batch: one launch over the row pairs of every sinogram; jobs[k]
@@ -505,8 +525,10 @@ __global__ void copy_rows_kernel(FilterLaunch a) {
   const int r = blockIdx.x, sl = blockIdx.y;
   const int N = a.N, W = a.W;
   const float *x = a.x + sl * a.x_slice_stride + (int64_t)r * W;
-  T *q = reinterpret_cast<T *>(a.q) + sl * a.q_slice_stride + (int64_t)r * a.Wp +
-         (a.off ? a.off : kRowOff);
+  const int es = a.quad ? kQuadSlices : 1;  // elements between samples
+  T *q = reinterpret_cast<T *>(a.q) + (a.quad ? (sl / kQuadSlices) * a.q_slice_stride + sl % kQuadSlices
+                                              : sl * a.q_slice_stride) +
+         ((int64_t)r * a.Wp + (a.off ? a.off : kRowOff)) * es;
   const float *ring = a.ring ? a.ring + (int64_t)sl * W : nullptr;
   auto xv = [&](int c) { return ring ? __fadd_rn(x[c], ring[c]) : x[c]; };
   __shared__ float red[32];
@@ -523,14 +545,18 @@ __global__ void copy_rows_kernel(FilterLaunch a) {
     if (threadIdx.x == 0) a.row_scale[(int64_t)sl * N + r] = s;
   }
   const float inv = 1.f / s;
-  for (int c = threadIdx.x; c < W; c += blockDim.x) q[c] = to_store<T>(xv(c) * inv);
+  float *dense = a.dense ? a.dense + ((int64_t)sl * N + r) * W : nullptr;
+  for (int c = threadIdx.x; c < W; c += blockDim.x) {
+    q[c * es] = to_store<T>(xv(c) * inv);
+    if (dense) dense[c] = xv(c);
+  }
   if (threadIdx.x == 0 && a.guard) {
-    q[-1] = to_store<T>(xv(0) * inv);
+    q[-es] = to_store<T>(xv(0) * inv);
     // the next row's first sample: read only where that row exists (on the
     // last row of the last slice x[W] lies past the end of the input)
     float nx = 0.f;
     if (a.store == 0 && r + 1 < N) nx = ring ? __fadd_rn(x[W], ring[0]) : x[W];
-    q[W] = to_store<T>(nx);
+    q[W * es] = to_store<T>(nx);
   }
 }
 
@@ -621,16 +647,18 @@ __global__ void unpad_kernel(const T *q, int64_t q_slice_stride, const float *ro
 // the flat sample r*W + k of the slice -- sample k - dr*W of row r + dr,
 // dr = floor(k / W) -- and 0 outside the slice's rows.  Reads only the data
 // columns, writes only the halo columns, so rows can be filled in any order.
-__global__ void halo_kernel(float *q, int64_t q_slice_stride, int N, int W, int Wp, int off) {
+// T: float, or float4 for the groups of the interleaved layout.
+template <typename T>
+__global__ void halo_kernel(T *q, int64_t q_slice_stride, int N, int W, int Wp, int off) {
   const int r = blockIdx.x, sl = blockIdx.y;
-  float *base = q + sl * q_slice_stride;
-  float *row = base + (int64_t)r * Wp;
+  T *base = q + sl * q_slice_stride;
+  T *row = base + (int64_t)r * Wp;
   for (int c = threadIdx.x; c < Wp; c += blockDim.x) {
     if (c >= off && c < off + W) continue;
     const int k = c - off;
     const int dr = k >= 0 ? k / W : -((-k + W - 1) / W);
     const int rr = r + dr, kk = k - dr * W;
-    row[c] = (rr >= 0 && rr < N) ? base[(int64_t)rr * Wp + off + kk] : 0.f;
+    row[c] = (rr >= 0 && rr < N) ? base[(int64_t)rr * Wp + off + kk] : T{};
   }
 }
 
@@ -654,6 +682,18 @@ cudaError_t launch_filter_t(const FilterLaunch &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+cudaError_t launch_filter_quad(const FilterLaunch &a, cudaStream_t st) {
+  const size_t smem = sizeof(float2) * (size_t)(a.P + a.P / 16);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        filter_quad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid(kQuadSlices * ((a.N + 1) / 2), (a.S + kQuadSlices - 1) / kQuadSlices);
+  filter_quad_kernel<<<grid, kFftThreads, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_filter_batch(const FilterLaunch *jobs_dev, const int *pair_begin_dev, int n_jobs,
@@ -672,7 +712,16 @@ cudaError_t launch_halo(float *q, int64_t q_slice_stride, int N, int W, int Wp, 
   return cudaGetLastError();
 }
 
+cudaError_t launch_halo_quad(float *q, int64_t q_group_stride, int N, int W, int Wp, int off, int S,
+                             cudaStream_t st) {
+  halo_kernel<<<dim3(N, (S + kQuadSlices - 1) / kQuadSlices), 256, 0, st>>>(
+      reinterpret_cast<float4 *>(q), q_group_stride, N, W, Wp, off);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_filter(const FilterLaunch &a, cudaStream_t st) {
+  if (a.quad && a.store != 0) return cudaErrorInvalidValue;
+  if (a.quad && a.contrast != 3) return launch_filter_quad(a, st);
   if (a.store == 1) return launch_filter_t<__half>(a, st);
   if (a.store == 2) return launch_filter_t<__nv_bfloat16>(a, st);
   return launch_filter_t<float>(a, st);

@@ -89,6 +89,9 @@ enum { CTAS_STORE_F32 = 0, CTAS_STORE_F16 = 1, CTAS_STORE_BF16 = 2 };
  * out; the call reports CTAS_E_TIMEOUT and the device stays usable.  (The
  * timeout path of the kernel: drain, error word, early return.) */
 #define CTAS_FLAG_TEST_TIMEOUT 0x200u
+/* Test aid: stacks of three or more slices go through the four-slice kernel
+ * however small they are (it otherwise takes stacks that fill the device). */
+#define CTAS_FLAG_GROUPS 0x400u
 
 typedef struct ctas_fbp_opts {
   uint32_t struct_size;   /* sizeof(ctas_fbp_opts); 0 is treated as "all defaults" */
