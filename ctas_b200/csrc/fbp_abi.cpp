@@ -239,12 +239,12 @@ void init_streams(ctas_fbp *h) {
   *h->err_host = 0;
 }
 
-// Whether stacks of this handle may go through the four-slice kernel: float32
-// rows, the reference's truncation on rows that serve it without branches
-// (sines >= 0, or the wide layout), and no tile asked for by id.
+// Whether stacks of this handle may go through the four-slice kernel: rows that serve
+// the index rule without branches (sines >= 0, or the reference's truncation on the wide
+// layout), and no tile asked for by id.  16-bit rows are expanded to float32 groups for it, a
+// bounded number at a time.
 bool quad_capable(const ctas_fbp *h) {
-  return h->store == CTAS_STORE_F32 && h->interp == CTAS_INTERP_TRUNC &&
-         (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
+  return h->interp == CTAS_INTERP_TRUNC && (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
          !ctas::bp_fast_tile_forced();
 }
 
@@ -261,6 +261,14 @@ int64_t quad_count(const ctas_fbp *h, int64_t S) {
 
 int64_t quad_groups(int64_t slices) { return (slices + ctas::kQuadSlices - 1) / ctas::kQuadSlices; }
 
+// Groups that the interleaved buffer holds: all of them for float32 rows, which the
+// filter stores there; for 16-bit rows as many as 512 MB take, expanded in turn.
+int64_t quad_resident(const ctas_fbp *h, int64_t groups) {
+  if (h->store == CTAS_STORE_F32) return groups;
+  const int64_t bytes = sizeof(float) * ctas::kQuadSlices * h->N * h->Wp;
+  return std::min(groups, std::max<int64_t>(1, ((int64_t)512 << 20) / bytes));
+}
+
 // First row of the interleaved buffer.
 float *quad_rows(const WorkSet &w) {
   return w.quad.as<float>() + ctas::kQuadSlices * ctas::kQuadSlack;
@@ -275,10 +283,10 @@ void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw) {
   // most slices that a launch of at most S leaves to the one-slice kernel: those below
   // the first count that forms groups, or a rest of two
   int64_t alone = S;
-  if (n4 > 0)
+  if (n4 > 0 && h->store == CTAS_STORE_F32)
     for (alone = 2; quad_count(h, alone + 1) == 0;) alone++;
   if (n4 > 0) {
-    const int64_t words = quad_groups(S) * N * h->Wp + 2 * ctas::kQuadSlack;
+    const int64_t words = quad_resident(h, quad_groups(S)) * N * h->Wp + 2 * ctas::kQuadSlack;
     if (w.quad.ensure(sizeof(float) * ctas::kQuadSlices * (size_t)words))
       cuda_check(cudaMemset(w.quad.p, 0, w.quad.bytes), "cudaMemset");
   }
@@ -346,8 +354,8 @@ const float *run_ring(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaSt
   return w.ring.as<float>();
 }
 
-// Filter S slices of x (device, dense S x N x W): the first quad_count() into w.quad,
-// the others into w.filt; densely into `dense` too, unless null (float32 store).
+// Filter S slices of x (device, dense S x N x W): with float32 rows the first
+// quad_count() into w.quad, all others into w.filt; densely into `dense` too, unless null (float32 store).
 void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t st,
                 float *dense = nullptr) {
   const float *ring = run_ring(h, x, S, w, st);
@@ -380,7 +388,7 @@ void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t
   a.ring = ring;
   a.off = (int)h->off;
   a.dense = dense;
-  const int64_t n4 = quad_count(h, S), rest = S - n4;
+  const int64_t n4 = h->store == CTAS_STORE_F32 ? quad_count(h, S) : 0, rest = S - n4;
   KernelTimer tm(h, CTAS_KERNEL_FILTER, st);
   if (n4 > 0) {
     ctas::FilterLaunch b = a;
@@ -452,19 +460,34 @@ void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, 
   const int64_t n4 = centers_dev ? 0 : quad_count(h, S);
   if (n4 > 0) {
     KernelTimer tm(h, CTAS_KERNEL_BACKPROJECT, st);
-    ctas::BpLaunch g = b;
-    g.q = quad_rows(w);
-    g.S = (int)n4;
-    const cudaError_t e = ctas::launch_bp_quad(g, st, (h->flags & CTAS_FLAG_CHECKED) != 0);
-    if (e != cudaSuccess)
-      cuda_check(e, (std::string("backprojection kernel: ") + ctas::bp_quad_error_detail()).c_str());
+    const int64_t step = ctas::kQuadSlices * quad_resident(h, quad_groups(n4));
+    for (int64_t s0 = 0; s0 < n4; s0 += step) {
+      ctas::BpLaunch g = b;
+      g.q = quad_rows(w);
+      g.S = (int)std::min(step, n4 - s0);
+      g.out = out + s0 * b.out_slice_stride;
+      if (h->store != CTAS_STORE_F32) {
+        cuda_check(ctas::launch_expand_quad(w.filt.as<char>() + elem_bytes(h->store) * s0 * h->N * h->Wp,
+                                            h->N * h->Wp, w.scale.as<float>() + s0 * h->N, h->store,
+                                            (int)h->N, (int)h->Wp, g.S, quad_rows(w), st),
+                   "expansion kernel");
+        h->launches += 1;
+      }
+      const cudaError_t e = ctas::launch_bp_quad(g, st, (h->flags & CTAS_FLAG_CHECKED) != 0);
+      if (e != cudaSuccess)
+        cuda_check(e, (std::string("backprojection kernel: ") + ctas::bp_quad_error_detail()).c_str());
+      h->launches += 1;
+    }
     tm.done();
-    h->launches += 1;
     h->last_kernel = 2;
     h->last_tile = -1;
     if (n4 == S) return;
     b.S = (int)(S - n4);
     b.out = out + n4 * b.out_slice_stride;
+    if (h->store != CTAS_STORE_F32) {  // all of the 16-bit rows are in w.filt
+      b.q = w.filt.as<char>() + elem_bytes(h->store) * n4 * h->N * h->Wp;
+      b.row_scale += n4 * h->N;
+    }
   }
   const bool fast = ctas::bp_fast_supported(b) &&
                     (h->interp == CTAS_INTERP_LINEAR || h->sines_nonneg || h->wide);
@@ -1142,7 +1165,7 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
     // four-slice groups are filtered into interleaved rows: the rows to write back are
     // stored densely beside them
-    const bool dense = wb && quad_count(h, C) > 0;
+    const bool dense = wb && h->store == CTAS_STORE_F32 && quad_count(h, C) > 0;
     for (auto &w : h->ws) {
       ensure_set(h, w, C, true);
       if (dense) w.dense.ensure(sizeof(float) * (size_t)(C * NW));

@@ -112,6 +112,11 @@ cudaError_t launch_halo(float *q, int64_t q_slice_stride, int N, int W, int Wp, 
 cudaError_t launch_halo_quad(float *q, int64_t q_group_stride, int N, int W, int Wp, int off, int S,
                              cudaStream_t st);
 
+// S slices of 16-bit padded rows (store 1 f16, 2 bf16) as interleaved float32 rows, a
+// group of four after another; the last group's missing slices repeat the last one.
+cudaError_t launch_expand_quad(const void *q, int64_t q_slice_stride, const float *row_scale,
+                               int store, int N, int Wp, int S, float *out, cudaStream_t st);
+
 struct BpLaunch {
   const void *q;             // padded filtered rows (see above)
   int interp;                // 0 reference truncation, 1 linear interpolation

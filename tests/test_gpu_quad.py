@@ -119,6 +119,24 @@ def test_stack_equals_single_calls(contrast, arc, ring):
         assert np.array_equal(_bits(rec.repeat(None, c)), _bits(single[0]))
 
 
+@pytest.mark.parametrize("store", [1, 2])
+@pytest.mark.parametrize("S,N,W", [(3, 40, 300), (7, 33, 97), (6, 64, 260)])
+def test_16bit_stack_equals_single_calls(S, N, W, store):
+    """Groups expanded from 16-bit rows: the bits of one call per slice, which converts
+    the same samples in the one-slice kernel."""
+    x = _rows(S, N, W, 5 * S)
+    x[1, ::3] *= 1e-3                       # rows of other scales
+    x[0, 5] = 0.0
+    with ct.CTrec((N, W), ct.Contrast.PHS, 180.0, ct.Filter("HANN"), store=store,
+                  flags=_lib.FLAG_GROUPS) as rec:
+        back = x.copy()
+        single = np.stack([rec.reconstruct(back[s], None, 1.5) for s in range(S)])
+        y = x.copy()
+        got = rec.reconstruct_stack(y, None, 1.5)
+    assert np.array_equal(_bits(got), _bits(single))
+    assert np.array_equal(_bits(y), _bits(back))
+
+
 def test_waits_run_out_and_context_survives():
     N, W = 120, 256
     q = _rows(4, N, W, 7)
