@@ -61,8 +61,6 @@ namespace {
 // SM (32 x 4 does not fit them: 16-bit stores then ran 24 % slower)
 constexpr int kChunk = 32;
 constexpr int kStages = 3;
-constexpr float kMagic = 12582912.0f;    // 1.5 * 2^23
-constexpr uint32_t kMagicBits = 0x4B400000u;
 
 thread_local char t_detail[160];  // last launch failure on this host thread
 
@@ -164,15 +162,6 @@ __device__ __forceinline__ float2 pair_to_f32(uint32_t w, __half) {
 }
 __device__ __forceinline__ float2 pair_to_f32(uint32_t w, __nv_bfloat16) {
   return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w));
-}
-
-__device__ __forceinline__ int window_start_linear(float sx, float cy, float t0, float ja,
-                                                   float jb, float ia, float ib, int align) {
-  const float a = fmaf(sx, ja, t0), b = fmaf(sx, jb, t0);
-  const float tmin = fminf(fminf(fmaf(cy, ia, a), fmaf(cy, ib, a)),
-                           fminf(fmaf(cy, ia, b), fmaf(cy, ib, b)));
-  const int lo = (int)floorf(tmin) - 2;
-  return lo & ~(align - 1);
 }
 
 // One slice as the tile routine sees it.

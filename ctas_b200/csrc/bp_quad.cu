@@ -27,6 +27,9 @@
 // The loop over projections is not unrolled: a pass is 130 instructions for each of 12
 // patterns and layouts, and twice that no longer stays in the instruction cache
 // (2398 us with 4 warps a CTA).  Half the pixels per thread, 24 warps an SM: 998 us.
+// Linear interpolation (an extension, FP64-derived projection bases) uses the same
+// layouts and patterns with two loads per sample: 397 instead of 980 us per slice of
+// 900 x 1536, bound by registers (its samples, differences and fractions).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -58,8 +61,10 @@ using QLarge = QTile<4, 2, 2, 96, 2>;  // 64 x 64, 16 pixels per thread
 using QSmall = QTile<4, 2, 1, 80, 3>;  // 32 x 64, 8 pixels per thread
 
 struct __align__(16) Param {
-  float sx, cy, base;  // sin, cos, c + ((1 - sin) - cos) * hp, times 2^-22
-  float m;             // 2 + (window word address - window start) * 2^-22
+  float sx, cy, base;  // sin, cos, c + ((1 - sin) - cos) * hp, times 2^-22; linear
+                       // interpolation: sin, cos, t0
+  float m;             // 2 + (window word address - window start) * 2^-22; linear
+                       // interpolation: the bits of the window's address bias
 };
 
 template <class TL> struct Layout {
@@ -219,6 +224,72 @@ __device__ __forceinline__ void project(const Param &p, const float2 (&cA)[2 * U
   }
 }
 
+// One projection with linear interpolation: u = t0 + sin j + cos i, k = floor(u),
+// q[k] + (u - k) (q[k+1] - q[k]).  Pixels that share a sample share its neighbour.
+template <int UB, bool ROW, int PAT, bool kCheck>
+__device__ __forceinline__ void project_linear(const Param &p, const float2 (&cA)[2 * UB],
+                                               const float2 (&cB)[UB], Acc<UB> &acc, uint32_t win,
+                                               uint32_t win_bytes, int *err) {
+  const uint32_t bias = __float_as_uint(p.m);
+  float2 rows[ROW ? 2 * UB : UB];  // t0 + sin j
+#pragma unroll
+  for (int q = 0; q < (ROW ? 2 * UB : UB); q++)
+    rows[q] = fma2_rn(both(p.sx), ROW ? cA[q] : cB[ROW ? 0 : q], both(p.base));
+#pragma unroll
+  for (int u = 0; u < UB; u++) {
+    uint32_t k[8];
+    float f[8];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      float2 v;
+      if constexpr (ROW) {
+        v = fma2_rn(both(p.cy), both(q < 2 ? cB[0].x : cB[0].y), rows[2 * u + (q & 1)]);
+      } else {
+        v = fma2_rn(both(p.cy), cA[q & 1], both(q < 2 ? rows[u].x : rows[u].y));
+      }
+      const float2 m = add2_rm(v, both(kMagic));
+      const float2 fl = add2_rn(m, both(-kMagic));
+      k[2 * q] = __float_as_uint(m.x);
+      k[2 * q + 1] = __float_as_uint(m.y);
+      f[2 * q] = __fsub_rn(v.x, fl.x);
+      f[2 * q + 1] = __fsub_rn(v.y, fl.y);
+    }
+    float2 w[8][2], d[8][2];  // samples and differences to the next ones
+    auto add = [&](int i, int h, float2 w0, float2 w1) {
+      float2 &o = *reinterpret_cast<float2 *>(&acc[u][i][h]);
+      o = add2_rn(o, fma2_rn(both(f[i]), w1, w0));
+    };
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      if (share(PAT, i).a >= 0) continue;
+      const uint32_t a = (k[i] << 4) + bias;
+      u64 x[2] = {0, 0}, y[2] = {0, 0};
+      if (!kCheck || a - win < win_bytes - 16) {
+        lds_quad(a, x);
+        lds_quad(a + 16, y);
+      } else {
+        atomicOr(err, 8);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const float2 y2 = *reinterpret_cast<float2 *>(&y[h]);
+        w[i][h] = *reinterpret_cast<float2 *>(&x[h]);
+        d[i][h] = add2_rn(y2, make_float2(-w[i][h].x, -w[i][h].y));
+        add(i, h, w[i][h], d[i][h]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int ia = share(PAT, i).a, ib = share(PAT, i).b;
+      if (ia < 0) continue;
+      if (kCheck && k[i] != k[ia] && k[i] != k[ib]) atomicOr(err, 8);
+      const bool same = k[i] == k[ia];
+#pragma unroll
+      for (int h = 0; h < 2; h++) add(i, h, same ? w[ia][h] : w[ib][h], same ? d[ia][h] : d[ib][h]);
+    }
+  }
+}
+
 // Row-major position of a thread's pixel in its 16 x 16 block; layout -1: the stores',
 // which put eight consecutive columns on eight lanes.
 __device__ __forceinline__ int place(int layout, int lane, int px) {
@@ -265,7 +336,7 @@ __device__ __forceinline__ void exchange(Acc<UB> &acc, float *buf, int lane, int
     }
 }
 
-template <class TL, bool kWide, bool kCheck>
+template <class TL, bool kLinear, bool kWide, bool kCheck>
 __global__ void __launch_bounds__(TL::THREADS, TL::MINB) bp_quad_kernel(BpLaunch a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Layout<TL> &sm = *reinterpret_cast<Layout<TL> *>(
@@ -337,17 +408,29 @@ __global__ void __launch_bounds__(TL::THREADS, TL::MINB) bp_quad_kernel(BpLaunch
     int x0 = 0;
     float tmin = 0.f;
     if (live) {
-      sc = a.tab[n];
-      const float base = ref_base(sc.x, sc.y, hp, c, a.rule);
-      x0 = window_start_trunc(sc.x, sc.y, base, geo(oj, pg, j0), geo(oj, pg, j0 + TL::TY - 1),
-                              geo(oi, pg, i0), geo(oi, pg, i0 + TL::TX - 1), c, 1, &tmin);
-      // off = window word address - x0, |off| < 2^22: M is exact
-      const int off = (int)(smem_u32(&sm.win[st][lane][0]) >> 4) - x0;
+      const float ja = geo(oj, pg, j0), jb = geo(oj, pg, j0 + TL::TY - 1);
+      const float ia = geo(oi, pg, i0), ib = geo(oi, pg, i0 + TL::TX - 1);
       Param p;
-      p.sx = __fmul_rn(sc.x, kTwoM22);
-      p.cy = __fmul_rn(sc.y, kTwoM22);
-      p.base = __fmul_rn(base, kTwoM22);
-      p.m = __fadd_rn(2.0f, __fmul_rn((float)off, kTwoM22));
+      if constexpr (kLinear) {
+        // u = t - 0.5, t0 formed in FP64
+        const double2 g = a.lin[n];
+        const double hc = (double)hp + (double)c;
+        p.sx = sc.x = (float)g.x;
+        p.cy = sc.y = (float)g.y;
+        p.base = (float)(hc * (1.0 - g.x) - g.y * (double)hp - 0.5);
+        x0 = window_start_linear(p.sx, p.cy, p.base, ja, jb, ia, ib, 1);
+        p.m = __uint_as_float(smem_u32(&sm.win[st][lane][0]) - 16u * (kMagicBits + (uint32_t)x0));
+      } else {
+        sc = a.tab[n];
+        const float base = ref_base(sc.x, sc.y, hp, c, a.rule);
+        x0 = window_start_trunc(sc.x, sc.y, base, ja, jb, ia, ib, c, 1, &tmin);
+        // off = window word address - x0, |off| < 2^22: M is exact
+        const int off = (int)(smem_u32(&sm.win[st][lane][0]) >> 4) - x0;
+        p.sx = __fmul_rn(sc.x, kTwoM22);
+        p.cy = __fmul_rn(sc.y, kTwoM22);
+        p.base = __fmul_rn(base, kTwoM22);
+        p.m = __fadd_rn(2.0f, __fmul_rn((float)off, kTwoM22));
+      }
       sm.par[st][lane] = p;
     }
     // the layout that most of the chunk's projections want
@@ -402,7 +485,7 @@ __global__ void __launch_bounds__(TL::THREADS, TL::MINB) bp_quad_kernel(BpLaunch
 #pragma unroll
   for (int e = 0; e < 16 * TL::UB; e++) (&acc[0][0][0])[e] = 0;
   float2 cA[2 * TL::UB], cB[TL::UB];
-  auto jc = [&](int j) { return __fsub_rn(geo(oj, pg, j), c); };
+  auto jc = [&](int j) { return kLinear ? geo(oj, pg, j) : __fsub_rn(geo(oj, pg, j), c); };
   auto coords = [&](int layout) {
     const int hi = place_of_lane(layout, lane) >> 3, lo = place_of_lane(layout, lane) & 7;
     auto slow = [&](int k) { return (layout & kMirror) ? 15 - (4 * hi + k) : 4 * hi + k; };
@@ -458,14 +541,18 @@ __global__ void __launch_bounds__(TL::THREADS, TL::MINB) bp_quad_kernel(BpLaunch
       const uint32_t rest = change >> k;
       const int end = rest ? k + __ffs(rest) : cnt;
       auto go = [&](auto row, auto pat, auto ng) {
-        constexpr bool ROW = decltype(row)::value, NEG = decltype(ng)::value;
+        constexpr bool ROW = decltype(row)::value;
+        [[maybe_unused]] constexpr bool NEG = decltype(ng)::value;
         constexpr int PAT = decltype(pat)::value;
         const Param *pp = &sm.par[st][k];
 #pragma unroll 1
         for (int n = k; n < end; n++) {
           const Param p = *pp++;
-          project<TL::UB, ROW, PAT, NEG, kCheck>(p, cA, cB, acc, lo_bits,
-                                         kCheck ? smem_u32(&sm.win[st][n][0]) : 0u, TL::BOX * 16, a.err);
+          const uint32_t win = kCheck ? smem_u32(&sm.win[st][n][0]) : 0u;
+          if constexpr (kLinear)
+            project_linear<TL::UB, ROW, PAT, kCheck>(p, cA, cB, acc, win, TL::BOX * 16, a.err);
+          else
+            project<TL::UB, ROW, PAT, NEG, kCheck>(p, cA, cB, acc, lo_bits, win, TL::BOX * 16, a.err);
         }
       };
       auto pick = [&](auto row, auto ng) {
@@ -509,9 +596,9 @@ __global__ void __launch_bounds__(TL::THREADS, TL::MINB) bp_quad_kernel(BpLaunch
     }
 }
 
-template <class TL, bool kWide, bool kCheck>
+template <class TL, bool kLinear, bool kWide, bool kCheck>
 cudaError_t launch(const BpLaunch &a, cudaStream_t st) {
-  auto kern = bp_quad_kernel<TL, kWide, kCheck>;
+  auto kern = bp_quad_kernel<TL, kLinear, kWide, kCheck>;
   const size_t smem = sizeof(Layout<TL>) + 128;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
@@ -529,8 +616,11 @@ cudaError_t launch(const BpLaunch &a, cudaStream_t st) {
 }
 
 template <class TL> cudaError_t launch_form(const BpLaunch &a, cudaStream_t st, bool check) {
-  if (a.wide) return check ? launch<TL, true, true>(a, st) : launch<TL, true, false>(a, st);
-  return check ? launch<TL, false, true>(a, st) : launch<TL, false, false>(a, st);
+  if (a.interp == 1)
+    return check ? launch<TL, true, false, true>(a, st) : launch<TL, true, false, false>(a, st);
+  if (a.wide)
+    return check ? launch<TL, false, true, true>(a, st) : launch<TL, false, true, false>(a, st);
+  return check ? launch<TL, false, false, true>(a, st) : launch<TL, false, false, false>(a, st);
 }
 
 }  // namespace
@@ -547,6 +637,7 @@ cudaError_t launch_bp_quad(const BpLaunch &a, cudaStream_t st, bool check) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (a.interp == 1 && a.wide) return cudaErrorInvalidValue;
   const int64_t tiles = (int64_t)((a.out_rows + QLarge::TY - 1) / QLarge::TY) *
                         ((a.out_cols + QLarge::TX - 1) / QLarge::TX) * ((a.S + 3) / 4);
   return 2 * tiles < 3 * sms ? launch_form<QSmall>(a, st, check) : launch_form<QLarge>(a, st, check);

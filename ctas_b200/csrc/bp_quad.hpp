@@ -8,7 +8,8 @@ namespace ctas {
 // Backprojects a.S slices of one geometry whose filtered rows are interleaved four
 // slices to a sample (kQuadSlices, fbp_kernels.hpp): a.q points at row 0, column 0,
 // with kQuadSlack samples allocated before it and behind the last row.  Reference
-// truncation, float32, every sine >= 0 or the wide layout, 0 < geo_p <= 1.
+// truncation, float32, every sine >= 0 or the wide layout, 0 < geo_p <= 1; or linear
+// interpolation of rows without guard columns, every sine >= 0.
 // `check`: every shared-memory read is bounds-checked (violations set bit 8 of
 // *a.err and read 0); for tests.
 // Two tiles: 64 x 64 from one and a half tiles per SM on, else 32 x 64 with half the

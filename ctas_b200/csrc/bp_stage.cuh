@@ -11,6 +11,8 @@ namespace ctas {
 namespace {
 
 constexpr uint32_t kWaitLimit = 1u << 22;
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr uint32_t kMagicBits = 0x4B400000u;
 constexpr float kTwoM22 = 2.384185791015625e-07f;  // 2^-22
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -116,6 +118,15 @@ __device__ __forceinline__ float2 mul2z_rn(float2 a, float2 b) {
   return r;
 }
 
+__device__ __forceinline__ float2 fma2_rn(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n .reg .b64 ra, rb, rc, rr;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
+      " mov.b64 rc, {%6, %7};\n fma.rn.f32x2 rr, ra, rb, rc;\n mov.b64 {%0, %1}, rr;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
 // x << 2 as a funnel shift of (x : lo) with lo < 2^30, so that it runs on the
 // integer ALU rather than as a multiply-add
 __device__ __forceinline__ uint32_t shl2_alu(uint32_t x, uint32_t lo) {
@@ -152,6 +163,15 @@ __device__ __forceinline__ int window_start_trunc(float sx, float cy, float base
   const float tmin = fminf(fminf(__fadd_rn(b0, d0), __fadd_rn(b0, d1)),
                            fminf(__fadd_rn(b1, d0), __fadd_rn(b1, d1)));
   if (tmin_out) *tmin_out = tmin;
+  const int lo = (int)floorf(tmin) - 2;
+  return lo & ~(align - 1);
+}
+
+__device__ __forceinline__ int window_start_linear(float sx, float cy, float t0, float ja,
+                                                   float jb, float ia, float ib, int align) {
+  const float a = fmaf(sx, ja, t0), b = fmaf(sx, jb, t0);
+  const float tmin = fminf(fminf(fmaf(cy, ia, a), fmaf(cy, ib, a)),
+                           fminf(fmaf(cy, ia, b), fmaf(cy, ib, b)));
   const int lo = (int)floorf(tmin) - 2;
   return lo & ~(align - 1);
 }

@@ -244,7 +244,7 @@ void init_streams(ctas_fbp *h) {
 // layout), and no tile asked for by id.  16-bit rows are expanded to float32 groups for it, a
 // bounded number at a time.
 bool quad_capable(const ctas_fbp *h) {
-  return h->interp == CTAS_INTERP_TRUNC && (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
+  return (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
          !ctas::bp_fast_tile_forced();
 }
 

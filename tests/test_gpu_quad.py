@@ -137,6 +137,28 @@ def test_16bit_stack_equals_single_calls(S, N, W, store):
     assert np.array_equal(_bits(y), _bits(back))
 
 
+@pytest.mark.parametrize("checked", [True, False])
+@pytest.mark.parametrize("S,N,W,c,store", [(3, 180, 256, 2.5, 0), (7, 33, 97, -30.25, 0),
+                                           (4, 61, 300, 0.0, 0), (8, 40, 1290, -7.5, 0),
+                                           (4, 90, 260, 1.25, 1), (4, 5, 33, 0.0, 0)])
+def test_linear_stack_vs_fp64_oracle(S, N, W, c, store, checked):
+    """Linear interpolation of given rows (FLT): within the one-slice kernel's bounds
+    against FP64 (relative RMSE 1e-5 float32, 2e-3 float16), and 0 outside the disc."""
+    x = np.linspace(-1, 1, W)
+    q = np.stack([np.exp(-(3 * x + 0.1 * s) ** 2)[None] * (1 + 0.3 * np.sin(np.arange(N) + s))[:, None]
+                  for s in range(S)]).astype(np.float32)
+    tab = O.angle_table_f64(180.0, N)
+    m = O.mask(W, c)
+    with ct.CTrec((N, W), ct.Contrast.FLT, 180.0, interp=1, store=store, checked=checked,
+                  flags=_lib.FLAG_GROUPS) as rec:
+        got = rec.reconstruct_stack(q.copy(), None, c)
+    for s in range(S):
+        want = O.bp_linear(q[s].astype(np.float64), tab, c, 1.0)
+        err = np.sqrt(np.mean((got[s][m] - want[m]) ** 2)) / np.sqrt(np.mean(want[m] ** 2))
+        assert err <= (1e-5 if store == 0 else 2e-3), s
+        assert (got[s][~m] == 0).all()
+
+
 def test_waits_run_out_and_context_survives():
     N, W = 120, 256
     q = _rows(4, N, W, 7)
