@@ -14,15 +14,30 @@
 //      tap ky's 128 x CK operand is the same box shifted by 16 ky rows, which
 //      keeps every operand start on a swizzle-atom boundary;
 //   B: the weights viewed as a 2-D array [cout][9 cin]; three NT x CK boxes per
-//      (kx, chunk), one per ky tap, placed one after another.
+//      (kx, chunk), one per ky tap, placed one after another -- loaded once and kept
+//      where all of them fit beside the input boxes, else with each input box.
 //
 // Persistent warp-specialised CTA (192 threads): warp 0 issues the TMA loads
-// into a ring of stages, one thread of warp 1 issues the MMAs (K = 16 each) and
-// releases each stage with tcgen05.commit, warps 2-5 drain the accumulator
-// (tcgen05.ld, bias, ReLU or ReLU mask, BF16) while the next tile accumulates in
-// the other half of the double-buffered tensor-memory accumulator.  Every wait is
-// bounded; on expiry the kernel records an error, drains its copies and MMAs,
-// frees its tensor memory and returns.
+// into a ring of stages, warp 1 issues the MMAs (K = 16 each) and releases each
+// stage with tcgen05.commit, warps 2-5 drain the accumulator (tcgen05.ld, bias, ReLU
+// or ReLU mask, BF16) through shared memory into TMA stores while the next tile
+// accumulates in another tensor-memory buffer.  Every wait is bounded; on expiry the
+// kernel records an error, drains its copies and MMAs, frees its tensor memory and
+// returns.
+//
+// What bounds it: the operands' shared-memory reads (128 x 16 and NT x 16 elements per
+// MMA: 48 clocks for N = 64, whose math takes 32) and, for 16 and 32 input channels,
+// the epilogue's latency per tile.  Measured steps, with the same outputs bit for bit:
+//   * the issuing warp stays converged and one elected lane issues each MMA, so that
+//     descriptors and counters live in uniform registers: a single thread took about 100
+//     clocks per MMA to form them.  With outputs through TMA stores (drain32) and a
+//     wait's limit loaded only when its first try fails, the row form below went from
+//     270 to 187 us on 64 -> 64 at 2 x 1024 x 1024, 528 to 403 on 96 -> 32 at 2048 x 2048,
+//     207 to 144 on 32 -> 32 and 180 to 125 on 16 -> 32;
+//   * resident weights, and all of tensor memory for the only CTA of an SM.
+// The tiled form with resident weights is faster still than the row form on 96 -> 32
+// (342 us) and 64 -> 64 (171), but adds a pixel's products in another order, which
+// changes the BF16 rounding of every layer after it.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -46,9 +61,9 @@ constexpr int kThreads = 192;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr int kMaxCout = 512;
 
+constexpr int kOutBytes = 32 * 32 * 2;  // 2 rows of 16 pixels x 32 channels
+
 struct TcArgs {
-  bf16 *y;
-  int y_cs, y_co;
   const bf16 *mask;
   int m_cs, m_co;
   const float *bias;
@@ -59,13 +74,18 @@ struct TcArgs {
   int64_t total;
   int cin;
   int kchunks;  // cin / CK
+  int stages;   // resident weights: stages of input boxes
   int *err;     // bit 0: a bounded wait ran out
 };
 
+// ST stages of (input box, weight boxes); ST = 0: the weights of all taps and chunks
+// stay in shared memory and a stage, of which there are TcArgs::stages, holds an input
+// box alone
 template <int CK, int NT, int ST> struct TcCfg {
+  static constexpr bool kResident = ST == 0;
   static constexpr int kABytes = 160 * CK * 2;     // 10 x 16 pixels x CK channels
   static constexpr int kBBytes = 3 * NT * CK * 2;  // three ky taps x NT x CK
-  static constexpr int kStage = kABytes + kBBytes;
+  static constexpr int kStage = kResident ? kABytes : kABytes + kBBytes;
   static constexpr int kRowB = CK * 2;             // bytes per operand row
   static constexpr int kSBO = 8 * kRowB;           // bytes between 8-row groups
   // descriptor layout type: 128 B / 64 B / 32 B swizzle
@@ -74,9 +94,18 @@ template <int CK, int NT, int ST> struct TcCfg {
   // per SM), so the MMAs run ahead of the epilogue on small tiles
   static constexpr int kAcc = 256 / NT >= 8 ? 8 : 256 / NT >= 4 ? 4 : 2;
   static constexpr uint32_t kCols = 256;
-  static constexpr int kBarOff = ST * kStage;
-  static constexpr int kBiasOff = kBarOff + 256;       // bias of all output channels
-  static constexpr int kSmem = kBiasOff + 4 * kMaxCout + 1024;  // + alignment slack
+  // barriers and two words, bias of all output channels, alignment slack
+  static constexpr int kMaxStages = kResident ? 8 : ST;
+  static constexpr int kBias = 512, kFixed = kBias + 4 * kMaxCout + 1024;
+  static_assert((2 * kMaxStages + 2 * kAcc + 2) * 8 + 8 <= kBias, "barriers run into the bias");
+  // output staging of each epilogue warp: buffers of 32 pixels x 32 channels, two where
+  // a tile fills several (96 -> 32 runs 418 instead of 342 us with a second one, which
+  // costs it a stage of input)
+  static constexpr int kOutBufs = NT == 32 ? 1 : 2;
+  static constexpr int kOut = 4 * kOutBufs * kOutBytes;
+  static constexpr int smem(int stages, int kchunks) {
+    return stages * kStage + (kResident ? 3 * kchunks * kBBytes : 0) + kOut + kFixed;
+  }
   static_assert(kABytes % 1024 == 0 && kBBytes % 1024 == 0, "stage alignment");
   static_assert(NT % 32 == 0 && NT >= 32 && NT <= 128, "UMMA N, epilogue pairs");
 };
@@ -117,8 +146,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 __device__ int g_test_stall = 0;
 __device__ uint32_t g_wait_limit = kWaitLimit;
 
-// bounded wait; false when the limit ran out
+// bounded wait; false when the limit ran out.  The limit is read after a first try:
+// its load would stand before every wait that is already over.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
   const uint32_t limit = __ldg(&g_wait_limit);
   for (uint32_t it = 0; it < limit; ++it)
     if (mbar_try_wait(bar, parity)) return true;
@@ -144,6 +175,17 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
+// shared -> global copy of a box, one bulk group
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, const void *src, int c0, int c1,
+                                             int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
+          reinterpret_cast<uint64_t>(map)),
+      "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(src))
+      : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -164,6 +206,24 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same by a whole converged warp, whose elected lane issues: descriptors and
+// loop counters stay warp-uniform, in uniform registers.
+__device__ __forceinline__ void tc_mma_w(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p, e;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+      " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_w(uint64_t *bar) {
+  asm volatile(
+      "{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+      " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(
+          smem_u32(bar))
       : "memory");
 }
 
@@ -188,6 +248,56 @@ template <class C> __device__ __forceinline__ uint64_t sdesc(uint32_t addr) {
          (C::kLayout << 61);
 }
 
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+
+// Epilogue step of one warp: 32 columns of its 32 accumulator rows (one pixel a lane) ->
+// bias, ReLU or mask -> BF16 in the staging buffer `so`, 64-byte rows in the 64-byte
+// swizzle of the store's tensor map.  Waits until at most PENDING earlier stores
+// still read their buffers.  A thread holds one pixel's channels, so its own global
+// stores would put every lane of a 16-byte store on another line, 32 wavefronts each.
+template <int PENDING>
+__device__ __forceinline__ void drain32(uint32_t taddr, const float *bias, const bf16 *mask, int relu,
+                                        uint8_t *so, int lane) {
+  // two 16-column loads in flight per wait
+  uint32_t r[2][16];
+  tmem_ld16(taddr, r[0]);
+  tmem_ld16(taddr + 16u, r[1]);
+  uint4 mk[4];
+  if (mask) {
+#pragma unroll
+    for (int h = 0; h < 4; h++) mk[h] = *reinterpret_cast<const uint4 *>(mask + 8 * h);
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
+  __syncwarp();
+  tmem_wait_ld();
+#pragma unroll
+  for (int h = 0; h < 4; h++) {  // 8 channels, one 16-byte word
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      v[j] = __uint_as_float(r[h >> 1][8 * (h & 1) + j]) + bias[8 * h + j];
+      if (relu) v[j] = fmaxf(v[j], 0.f);
+    }
+    if (mask) {
+      const bf16 *mm = reinterpret_cast<const bf16 *>(&mk[h]);
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        if (!(__bfloat162float(mm[j]) > 0.f)) v[j] = 0.f;
+    }
+    uint4 o;
+    o.x = pack_bf16(v[0], v[1]);
+    o.y = pack_bf16(v[2], v[3]);
+    o.z = pack_bf16(v[4], v[5]);
+    o.w = pack_bf16(v[6], v[7]);
+    *reinterpret_cast<uint4 *>(so + lane * 64 + ((h ^ ((lane >> 1) & 3)) << 4)) = o;
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+}
+
 struct Tile {
   int b, ty, tx, nt;
 };
@@ -203,34 +313,37 @@ __device__ __forceinline__ Tile decode(const TcArgs &a, int64_t t) {
   return r;
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t *>(&v);
-}
 
 template <int CK, int NT, int ST>
 __global__ void __launch_bounds__(kThreads, 1)
     conv_tc_kernel(const __grid_constant__ CUtensorMap amap,
-                   const __grid_constant__ CUtensorMap bmap, TcArgs a) {
+                   const __grid_constant__ CUtensorMap bmap,
+                   const __grid_constant__ CUtensorMap ymap, TcArgs a) {
   using C = TcCfg<CK, NT, ST>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *base = smem_raw + pad;
-  uint64_t *full = reinterpret_cast<uint64_t *>(base + C::kBarOff);
-  uint64_t *empty = full + ST;
-  uint64_t *acc_full = empty + ST;  // [kAcc]
+  const int nst = C::kResident ? a.stages : ST;
+  uint8_t *wts = base + nst * C::kStage;  // resident weights: [chunk][kx][ky] blocks
+  uint8_t *outs = wts + (C::kResident ? 3 * a.kchunks * C::kBBytes : 0);
+  uint8_t *bars = outs + C::kOut;
+  uint64_t *full = reinterpret_cast<uint64_t *>(bars);
+  uint64_t *empty = full + nst;
+  uint64_t *acc_full = empty + nst;  // [kAcc]
   uint64_t *acc_empty = acc_full + C::kAcc;
   uint64_t *drain = acc_empty + C::kAcc;
-  uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
+  uint64_t *wfull = drain + 1;  // resident weights have landed
+  uint32_t *s_tmem = reinterpret_cast<uint32_t *>(wfull + 1);
   volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
-  float *s_bias = reinterpret_cast<float *>(base + C::kBiasOff);
+  float *s_bias = reinterpret_cast<float *>(bars + C::kBias);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < ST; s++) {
+    for (int s = 0; s < nst; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
+    mbar_init(wfull, 1);
     for (int i = 0; i < C::kAcc; i++) {
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_empty[i], 128);
@@ -263,6 +376,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       int stage = 0;
       uint32_t ph = 0;
       uint32_t issued = 0, last_par = 0;  // per-stage bits: used / parity of last issue
+      if constexpr (C::kResident) {
+        mbar_expect_tx(wfull, (uint32_t)(3 * a.kchunks * C::kBBytes));
+        for (int i = 0; i < 9 * a.kchunks; i++) {  // block (chunk, kx, ky)
+          const int ky = i % 3, kx = i / 3 % 3, kc = i / 9;
+          tma_load_2d(wts + i * NT * C::kRowB, &bmap, (ky * 3 + kx) * a.cin + kc * CK, 0, wfull);
+        }
+      }
       for (int64_t t = blockIdx.x; t < a.total && !*s_abort; t += gridDim.x) {
         const Tile tl = decode(a, t);
         for (int ks = 0; ks < ksteps; ks++) {
@@ -274,83 +394,96 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           uint8_t *sa = base + stage * C::kStage;
           mbar_expect_tx(&full[stage], (uint32_t)C::kStage);
-          if (!(__ldg(&g_test_stall) && t == blockIdx.x && ks == 0)) {
+          if (!(t == blockIdx.x && ks == 0 && __ldg(&g_test_stall))) {
             tma_load_4d(sa, &amap, kc * CK, tl.tx * 16 + kx - 1, tl.ty * 8 - 1, tl.b, &full[stage]);
+            if constexpr (!C::kResident) {
 #pragma unroll
-            for (int ky = 0; ky < 3; ky++)
-              tma_load_2d(sa + C::kABytes + ky * NT * C::kRowB, &bmap,
-                          (ky * 3 + kx) * a.cin + kc * CK, tl.nt * NT, &full[stage]);
+              for (int ky = 0; ky < 3; ky++)
+                tma_load_2d(sa + C::kABytes + ky * NT * C::kRowB, &bmap,
+                            (ky * 3 + kx) * a.cin + kc * CK, tl.nt * NT, &full[stage]);
+            }
           }
           issued |= 1u << stage;
           last_par = (last_par & ~(1u << stage)) | (ph << stage);
-          if (++stage == ST) {
+          if (++stage == nst) {
             stage = 0;
             ph ^= 1;
           }
         }
       }
       // every issued copy has landed before the CTA may exit
-      for (int s = 0; s < ST; s++)
+      for (int s = 0; s < nst; s++)
         if ((issued >> s) & 1u)
           if (!mbar_wait(&full[s], (last_par >> s) & 1u)) atomicOr(a.err, 1);
+      if (C::kResident && !mbar_wait(wfull, 0)) atomicOr(a.err, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------ MMA issuer
+    {
+      // ------------------------------------------------ MMA issuer (whole warp)
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) |
                                  ((uint32_t)(128 >> 4) << 24);
       int stage = 0;
       uint32_t ph = 0;
       int acc = 0;
       uint32_t acc_ph = 0;
-      for (int64_t t = blockIdx.x; t < a.total && !*s_abort; t += gridDim.x) {
-        if (!mbar_wait(&acc_empty[acc], acc_ph ^ 1)) {
-          atomicOr(a.err, 1);
-          *s_abort = 1;
+      if (C::kResident && !__all_sync(0xffffffffu, mbar_wait(wfull, 0)) && lane == 0) {
+        atomicOr(a.err, 1);
+        *s_abort = 1;
+      }
+      __syncwarp();
+      for (int64_t t = blockIdx.x; t < a.total && !__shfl_sync(0xffffffffu, *s_abort, 0); t += gridDim.x) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_ph ^ 1))) {
+          if (lane == 0) {
+            atomicOr(a.err, 1);
+            *s_abort = 1;
+          }
           break;
         }
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(acc * NT);
         bool ok = true;
         for (int ks = 0; ks < ksteps; ks++) {
-          if (!mbar_wait(&full[stage], ph)) {
-            atomicOr(a.err, 1);
-            *s_abort = 1;
+          if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], ph))) {
+            if (lane == 0) {
+              atomicOr(a.err, 1);
+              *s_abort = 1;
+            }
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(base + stage * C::kStage);
-          const uint64_t da = sdesc<C>(sa), db = sdesc<C>(sa + C::kABytes);
+          const uint64_t da = sdesc<C>(sa),
+                         db = sdesc<C>(C::kResident ? smem_u32(wts) + ks * C::kBBytes : sa + C::kABytes);
 #pragma unroll
           for (int ky = 0; ky < 3; ky++)
 #pragma unroll
             for (int kk = 0; kk < CK / 16; kk++)
-              tc_mma(d, da + (uint64_t)((ky * 16 * C::kRowB + kk * 32) >> 4),
+              tc_mma_w(d, da + (uint64_t)((ky * 16 * C::kRowB + kk * 32) >> 4),
                      db + (uint64_t)((ky * NT * C::kRowB + kk * 32) >> 4), idesc,
                      (ks | ky | kk) != 0 ? 1u : 0u);
-          tc_commit(&empty[stage]);  // the stage is free once these MMAs have read it
-          if (++stage == ST) {
+          tc_commit_w(&empty[stage]);  // the stage is free once these MMAs have read it
+          if (++stage == nst) {
             stage = 0;
             ph ^= 1;
           }
         }
         if (!ok) break;
-        tc_commit(&acc_full[acc]);
+        tc_commit_w(&acc_full[acc]);
         if (++acc == C::kAcc) {
           acc = 0;
           acc_ph ^= 1;
         }
       }
       // all MMAs of this thread complete before tensor memory is released
-      tc_commit(drain);
+      tc_commit_w(drain);
       if (!mbar_wait(drain, 0)) atomicOr(a.err, 1);
     }
   } else {
     // ---------------------------------------------------- epilogue (warps 2-5)
     const int q = warp & 3;  // tensor-memory lane quarter this warp may access
     const int m = q * 32 + lane;
-    int acc = 0;
+    int acc = 0, turn = 0;
     uint32_t acc_ph = 0;
     for (int64_t t = blockIdx.x; t < a.total; t += gridDim.x) {
       // warp-uniform decisions: the tensor-memory loads below are warp-collective
@@ -366,49 +499,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       const Tile tl = decode(a, t);
       const int yy = tl.ty * 8 + (m >> 4), xx = tl.tx * 16 + (m & 15);
       const int64_t pix = ((int64_t)tl.b * a.H + yy) * a.W + xx;
-      bf16 *yp = a.y + pix * a.y_cs + a.y_co + tl.nt * NT;
       const bf16 *mp = a.mask ? a.mask + pix * a.m_cs + a.m_co + tl.nt * NT : nullptr;
       const float *bp = s_bias + tl.nt * NT;
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NT);
 #pragma unroll 1
-      for (int c0 = 0; c0 < NT; c0 += 32) {
-        // two 16-column loads in flight per wait
-        uint32_t r[2][16];
-        tmem_ld16(taddr + (uint32_t)c0, r[0]);
-        tmem_ld16(taddr + (uint32_t)c0 + 16u, r[1]);
-        tmem_wait_ld();
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int cc = c0 + 16 * h;
-          float v[16];
-#pragma unroll
-          for (int j = 0; j < 16; j++) {
-            v[j] = __uint_as_float(r[h][j]) + bp[cc + j];
-            if (a.relu) v[j] = fmaxf(v[j], 0.f);
-          }
-          if (mp) {
-            const uint4 m0 = *reinterpret_cast<const uint4 *>(mp + cc);
-            const uint4 m1 = *reinterpret_cast<const uint4 *>(mp + cc + 8);
-            const bf16 *mm0 = reinterpret_cast<const bf16 *>(&m0);
-            const bf16 *mm1 = reinterpret_cast<const bf16 *>(&m1);
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-              if (!(__bfloat162float(mm0[j]) > 0.f)) v[j] = 0.f;
-              if (!(__bfloat162float(mm1[j]) > 0.f)) v[8 + j] = 0.f;
-            }
-          }
-          uint4 o0, o1;
-          o0.x = pack_bf16(v[0], v[1]);
-          o0.y = pack_bf16(v[2], v[3]);
-          o0.z = pack_bf16(v[4], v[5]);
-          o0.w = pack_bf16(v[6], v[7]);
-          o1.x = pack_bf16(v[8], v[9]);
-          o1.y = pack_bf16(v[10], v[11]);
-          o1.z = pack_bf16(v[12], v[13]);
-          o1.w = pack_bf16(v[14], v[15]);
-          *reinterpret_cast<uint4 *>(yp + cc) = o0;
-          *reinterpret_cast<uint4 *>(yp + cc + 8) = o1;
-        }
+      for (int c0 = 0; c0 < NT; c0 += 32, turn ^= 1) {
+        uint8_t *so = outs + (C::kOutBufs == 2 ? 2 * q + turn : q) * kOutBytes;
+        drain32<C::kOutBufs - 1>(taddr + (uint32_t)c0, bp + c0, mp ? mp + c0 : nullptr, a.relu, so, lane);
+        if (lane == 0) tma_store_4d(&ymap, so, tl.nt * NT + c0, tl.tx * 16, tl.ty * 8 + 2 * q, tl.b);
       }
       tc_fence_before();
       mbar_arrive(&acc_empty[acc]);
@@ -417,6 +515,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         acc_ph ^= 1;
       }
     }
+    // the staging buffers are read before the CTA may exit
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   tc_fence_before();
@@ -450,6 +550,23 @@ bool make_act_map(const ConvArgs &a, int ck, CUtensorMap *map) {
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16 *>(a.x + a.x_co), dims,
              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(ck),
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+         CUDA_SUCCESS;
+}
+
+// outputs: (cout, W, H, B) of the channel slice; box {32, bw, bh, 1}, bw * bh = 32
+bool make_out_map(const ConvArgs &a, int bw, int bh, CUtensorMap *map) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return false;
+  std::memset(map, 0, sizeof(*map));
+  const cuuint64_t dims[4] = {(cuuint64_t)a.cout, (cuuint64_t)a.W, (cuuint64_t)a.H,
+                              (cuuint64_t)a.B};
+  const cuuint64_t cs = (cuuint64_t)a.y_cs * 2;
+  const cuuint64_t strides[3] = {cs, cs * (cuuint64_t)a.W, cs * (cuuint64_t)a.W * a.H};
+  const cuuint32_t box[4] = {32u, (cuuint32_t)bw, (cuuint32_t)bh, 1u};
+  const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, a.y + a.y_co, dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
          CUDA_SUCCESS;
 }
@@ -520,12 +637,10 @@ int sm_count() {
 template <int CK, int NT, int ST>
 cudaError_t launch_cfg(const ConvArgs &a, cudaStream_t st) {
   using C = TcCfg<CK, NT, ST>;
-  CUtensorMap amap, bmap;
-  if (!make_act_map(a, CK, &amap) || !make_wt_map(a, CK, NT, &bmap)) return cudaErrorInvalidValue;
+  CUtensorMap amap, bmap, ymap;
+  if (!make_act_map(a, CK, &amap) || !make_wt_map(a, CK, NT, &bmap) || !make_out_map(a, 16, 2, &ymap))
+    return cudaErrorInvalidValue;
   TcArgs t{};
-  t.y = a.y;
-  t.y_cs = a.y_cs;
-  t.y_co = a.y_co;
   t.mask = a.mask;
   t.m_cs = a.m_cs;
   t.m_co = a.m_co;
@@ -545,7 +660,15 @@ cudaError_t launch_cfg(const ConvArgs &a, cudaStream_t st) {
   // no more CTAs per SM than tensor memory holds (512 columns): pad the
   // shared-memory request so that one more would not fit
   const int per_sm = 512 / (int)C::kCols;
-  const int smem = std::max(C::kSmem, 232448 / (per_sm + 1) + 1024);
+  t.stages = ST;
+  if (C::kResident) {
+    // two CTAs per SM where three stages fit beside the weights, else one
+    const int half = (233472 / 2 - 1024 - C::smem(0, t.kchunks)) / C::kStage;
+    const int all = (232448 - C::smem(0, t.kchunks)) / C::kStage;
+    t.stages = std::min(C::kMaxStages, half >= 3 ? half : all);
+    if (t.stages < 3) return cudaErrorInvalidValue;
+  }
+  const int smem = std::max(C::smem(t.stages, t.kchunks), 232448 / (per_sm + 1) + 1024);
   e = cudaFuncSetAttribute(conv_tc_kernel<CK, NT, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem);
   if (e != cudaSuccess) return e;
@@ -555,11 +678,19 @@ cudaError_t launch_cfg(const ConvArgs &a, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   const int occ = occupancy(conv_tc_kernel<CK, NT, ST>, smem, per_sm);
   const int64_t grid = std::min<int64_t>(t.total, (int64_t)sm_count() * occ);
-  conv_tc_kernel<CK, NT, ST><<<(unsigned)grid, kThreads, smem, st>>>(amap, bmap, t);
+  conv_tc_kernel<CK, NT, ST><<<(unsigned)grid, kThreads, smem, st>>>(amap, bmap, ymap, t);
   return cudaGetLastError();
 }
 
+// Whether the weights of all nine taps fit beside three input boxes (64 -> 128, 128 -> 64
+// and the layers below on rows that the row form does not take): the CTAs then read
+// them once instead of per tile.  64 -> 128 at 2 x 512 x 512 91 -> 70 us.
+template <int CK, int NT> bool resident_fits(const ConvArgs &a) {
+  return a.cout == NT && TcCfg<CK, NT, 0>::smem(3, a.cin / CK) <= 232448;
+}
+
 template <int CK, int NT> cudaError_t launch_ck_nt(const ConvArgs &a, cudaStream_t st) {
+  if (resident_fits<CK, NT>(a)) return launch_cfg<CK, NT, 0>(a, st);
   constexpr int kStage = 160 * CK * 2 + 3 * NT * CK * 2;
   constexpr int kSt = (96 * 1024) / kStage < 2 ? 2 : (96 * 1024) / kStage > 6 ? 6 : (96 * 1024) / kStage;
   return launch_cfg<CK, NT, kSt>(a, st);
@@ -593,10 +724,9 @@ constexpr int kRowPx = 130;                    // 128 output pixels + 2 halo
 constexpr int kRowChunkBytes = 17 * 1024;      // 130 x 128 B, padded to the 1 KB atom
 constexpr int kRowMaxSlots = 8;
 constexpr int kMaxAcc = 8;
+constexpr int kRowOut = 4 * 2 * kOutBytes;     // two staging buffers per epilogue warp
 
 struct RowArgs {
-  bf16 *y;
-  int y_cs, y_co;
   const bf16 *mask;
   int m_cs, m_co;
   const float *bias;
@@ -637,13 +767,15 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t addr) {
 
 template <int CIN>
 __global__ void __launch_bounds__(kThreads, 1)
-    conv_row_kernel(const __grid_constant__ CUtensorMap amap, RowArgs a) {
+    conv_row_kernel(const __grid_constant__ CUtensorMap amap,
+                    const __grid_constant__ CUtensorMap ymap, RowArgs a) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *base = smem_raw + pad;
   uint8_t *slots = base;                                   // input-row ring (1 KB atoms)
   uint8_t *wsm = base + a.nslots * a.slot_bytes;           // weights
-  float *s_bias = reinterpret_cast<float *>(wsm + a.wbytes);
+  uint8_t *outs = wsm + a.wbytes;                          // output staging
+  float *s_bias = reinterpret_cast<float *>(outs + kRowOut);
   uint64_t *row_full = reinterpret_cast<uint64_t *>(s_bias + kMaxCout);
   uint64_t *row_empty = row_full + kRowMaxSlots;
   uint64_t *acc_full = row_empty + kRowMaxSlots;  // [kMaxAcc]
@@ -724,7 +856,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           uint8_t *dst = slots + slot * a.slot_bytes;
           mbar_expect_tx(&row_full[slot], row_bytes);
-          if (!(__ldg(&g_test_stall) && j == 0))
+          if (!(j == 0 && __ldg(&g_test_stall)))
             for (int c = 0; c < chunks; c++)
               tma_load_4d(dst + c * kRowChunkBytes, &amap, c * 64, sx * 128 - 1, yi, b,
                           &row_full[slot]);
@@ -738,8 +870,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (!mbar_wait(&row_full[s], (last_par >> s) & 1u)) atomicOr(a.err, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------ MMA issuer
+    {
+      // ------------------------------------------------ MMA issuer (whole warp)
       // Input-row stationary: input row yi feeds output rows yi - 1, yi, yi + 1
       // (taps ky = 2, 1, 0), whose accumulators are consecutive blocks of cout
       // columns in a ring of nacc blocks; per (kx, 16-channel step) one MMA with
@@ -775,21 +907,24 @@ __global__ void __launch_bounds__(kThreads, 1)
       };
       uint32_t j0 = 0, o0 = 0;
       bool ok = true;
-      for (int64_t t = blockIdx.x; t < a.total && ok && !*s_abort; t += gridDim.x) {
+      for (int64_t t = blockIdx.x; t < a.total && ok && !__shfl_sync(0xffffffffu, *s_abort, 0);
+           t += gridDim.x) {
         const int64_t r = t / a.strips_x;
         const int sy = (int)(r % a.strips_y);
         const int r0 = sy * a.strip_h, r1 = min(r0 + a.strip_h, a.H);
         for (int yi = r0 - 1; yi <= r1 && ok; yi++) {
           const uint32_t jl = j0 + (uint32_t)(yi - r0 + 1);  // load index of input row yi
-          ok = mbar_wait(&row_full[jl % (uint32_t)ns], (jl / (uint32_t)ns) & 1u);
+          ok = __all_sync(0xffffffffu, mbar_wait(&row_full[jl % (uint32_t)ns], (jl / (uint32_t)ns) & 1u));
           const int lo = max(yi - 1, r0), hi = min(yi + 1, r1 - 1);
           const bool fresh = (yi + 1 <= r1 - 1);  // row yi + 1 starts here
           const uint32_t olo = o0 + (uint32_t)(lo - r0), ohi = o0 + (uint32_t)(hi - r0);
           if (ok && fresh)
-            ok = mbar_wait(&acc_empty[ohi % R], ((ohi / R) & 1u) ^ 1u);
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[ohi % R], ((ohi / R) & 1u) ^ 1u));
           if (!ok) {
-            atomicOr(a.err, 1);
-            *s_abort = 1;
+            if (lane == 0) {
+              atomicOr(a.err, 1);
+              *s_abort = 1;
+            }
             break;
           }
           tc_fence_after();
@@ -818,27 +953,27 @@ __global__ void __launch_bounds__(kThreads, 1)
                                    (uint32_t)((st % kSteps) * 2));
               if (kx == 0 && st == 0 && fresh) {
                 for (int q = 0; q < nhead; q++)
-                  tc_mma(head[q].d, a_op, b_op + head[q].boff, head[q].idesc, q < nacc_head ? 1u : 0u);
+                  tc_mma_w(head[q].d, a_op, b_op + head[q].boff, head[q].idesc, q < nacc_head ? 1u : 0u);
               } else {
-                tc_mma(all[0].d, a_op, b_op + all[0].boff, all[0].idesc, 1u);
-                if (nall > 1) tc_mma(all[1].d, a_op, b_op + all[1].boff, all[1].idesc, 1u);
+                tc_mma_w(all[0].d, a_op, b_op + all[0].boff, all[0].idesc, 1u);
+                if (nall > 1) tc_mma_w(all[1].d, a_op, b_op + all[1].boff, all[1].idesc, 1u);
               }
             }
-          tc_commit(&row_empty[jl % (uint32_t)ns]);       // input row yi is done
-          if (yi - 1 >= r0) tc_commit(&acc_full[olo % R]);  // output row yi - 1 is complete
+          tc_commit_w(&row_empty[jl % (uint32_t)ns]);       // input row yi is done
+          if (yi - 1 >= r0) tc_commit_w(&acc_full[olo % R]);  // output row yi - 1 is complete
         }
         if (!ok) break;
         j0 += (uint32_t)(r1 - r0) + 2u;
         o0 += (uint32_t)(r1 - r0);
       }
-      tc_commit(drain);
+      tc_commit_w(drain);
       if (!mbar_wait(drain, 0)) atomicOr(a.err, 1);
     }
   } else {
     // ---------------------------------------------------- epilogue (warps 2-5)
     const int q = warp & 3;
     const int m = q * 32 + lane;
-    int acc = 0;
+    int acc = 0, turn = 0;
     uint32_t acc_ph = 0;
     bool stop = false;
     for (int64_t t = blockIdx.x; t < a.total && !stop; t += gridDim.x) {
@@ -858,47 +993,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tc_fence_after();
         const int64_t pix = ((int64_t)b * a.H + y) * a.W + sx * 128 + m;
-        bf16 *yp = a.y + pix * a.y_cs + a.y_co;
         const bf16 *mp = a.mask ? a.mask + pix * a.m_cs + a.m_co : nullptr;
         const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * cout);
 #pragma unroll 1
-        for (int c0 = 0; c0 < cout; c0 += 32) {
-          uint32_t rr[2][16];
-          tmem_ld16(taddr + (uint32_t)c0, rr[0]);
-          tmem_ld16(taddr + (uint32_t)c0 + 16u, rr[1]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int cc = c0 + 16 * h;
-            float v[16];
-#pragma unroll
-            for (int jx = 0; jx < 16; jx++) {
-              v[jx] = __uint_as_float(rr[h][jx]) + s_bias[cc + jx];
-              if (a.relu) v[jx] = fmaxf(v[jx], 0.f);
-            }
-            if (mp) {
-              const uint4 m0 = *reinterpret_cast<const uint4 *>(mp + cc);
-              const uint4 m1 = *reinterpret_cast<const uint4 *>(mp + cc + 8);
-              const bf16 *mm0 = reinterpret_cast<const bf16 *>(&m0);
-              const bf16 *mm1 = reinterpret_cast<const bf16 *>(&m1);
-#pragma unroll
-              for (int jx = 0; jx < 8; jx++) {
-                if (!(__bfloat162float(mm0[jx]) > 0.f)) v[jx] = 0.f;
-                if (!(__bfloat162float(mm1[jx]) > 0.f)) v[8 + jx] = 0.f;
-              }
-            }
-            uint4 o0, o1;
-            o0.x = pack_bf16(v[0], v[1]);
-            o0.y = pack_bf16(v[2], v[3]);
-            o0.z = pack_bf16(v[4], v[5]);
-            o0.w = pack_bf16(v[6], v[7]);
-            o1.x = pack_bf16(v[8], v[9]);
-            o1.y = pack_bf16(v[10], v[11]);
-            o1.z = pack_bf16(v[12], v[13]);
-            o1.w = pack_bf16(v[14], v[15]);
-            *reinterpret_cast<uint4 *>(yp + cc) = o0;
-            *reinterpret_cast<uint4 *>(yp + cc + 8) = o1;
-          }
+        for (int c0 = 0; c0 < cout; c0 += 32, turn ^= 1) {
+          uint8_t *so = outs + (2 * q + turn) * kOutBytes;
+          drain32<1>(taddr + (uint32_t)c0, s_bias + c0, mp ? mp + c0 : nullptr, a.relu, so, lane);
+          if (lane == 0) tma_store_4d(&ymap, so, c0, sx * 128 + q * 32, y, b);
         }
         tc_fence_before();
         mbar_arrive(&acc_empty[acc]);
@@ -908,6 +1009,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
+    // the staging buffers are read before the CTA may exit
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   tc_fence_before();
@@ -918,8 +1021,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                  : "memory");
 }
 
-constexpr int kRowSmemFixed = 4 * kMaxCout + (2 * kRowMaxSlots + 2 * kMaxAcc + 1) * 8 + 16 + 1024;  // bias, barriers, slack
-constexpr int kRowSmemMax = 232448;
+constexpr int kRowSmemFixed = kRowOut + 4 * kMaxCout + (2 * kRowMaxSlots + 2 * kMaxAcc + 1) * 8 + 16 + 1024;  // bias, barriers, slack
+constexpr int kRowSmemMax = 232448, kRowSmemHalf = 233472 / 2 - 1024;
 
 // resident weights of the row form: 9 taps x cout rows x cin channels
 int row_wbytes(const ConvArgs &a) { return 9 * a.cin * a.cout * 2; }
@@ -957,9 +1060,12 @@ bool make_row_map(const ConvArgs &a, CUtensorMap *map) {
 // nine taps, into five tensor-memory accumulators.  The pixel blocks are split over
 // CTAs, which add their sums to dw.
 //
-// Bound by the operands' shared-memory reads (6 KB, 48 clocks per MMA whose math
-// takes 32).  One tap per CTA, M = 128 output channels, read dy and x from L2 once
-// per tap and was bound by that: 823 us for 64 -> 64 channels on 2 x 1024 x 1024.
+// Where nine-tap CTAs would fill less than half of the device, a CTA has the taps of
+// one kx.  Bound by the operands' shared-memory reads (6 KB, 48 clocks per MMA whose
+// math takes 32) and the issue of MMAs that short (70 clocks).  One tap per CTA, M = 128
+// output channels, read dy and x from L2 once per tap and was bound by that: 64 -> 64 at
+// 2 x 1024 x 1024 830 us, now 284; 32 -> 32 at 4 x 512 x 512 422 and 135, 192 -> 64 at
+// 2 x 512 x 512 448 and 218, 128 -> 128 at 4 x 256 x 256 129 and 95.
 struct WgTcArgs {
   float *dw;
   int cin, cout;
@@ -979,40 +1085,49 @@ __device__ __forceinline__ uint64_t sdesc_mn128(uint32_t addr, uint32_t lbo) {
 
 constexpr int kWgRow = 16 * 128;          // 16 pixels x 64 channels x 2 B
 constexpr int kWgBox = 10 * kWgRow;       // one kx: rows -1 .. 8
-constexpr int kWgStage = 3 * kWgBox + 8 * kWgRow;  // x boxes, then dy
-constexpr int kWgStages = 2;
-constexpr int kWgAcc = 5;
-constexpr int kWgSmem = kWgStages * kWgStage + 256 + 1024;  // + barriers, alignment slack
-// taps (3 ky + kx) of the lower and upper half of each accumulator
-__device__ __forceinline__ int wg_tap(int acc, int half) {
-  return acc < 3 ? 3 * half + acc : acc == 3 ? 6 + half : half == 0 ? 8 : -1;
-}
+// G = 1: a CTA has all nine taps; G = 3: those of one kx
+template <int G> struct WgCfg {
+  static constexpr int kBoxes = 3 / G, kAcc = G == 1 ? 5 : 2, kStages = G == 1 ? 2 : 3;
+  static constexpr uint32_t kCols = G == 1 ? 512 : 128;
+  static constexpr int kStage = kBoxes * kWgBox + 8 * kWgRow;  // x boxes, then dy
+  static constexpr int kSmem = kStages * kStage + 256 + 1024;  // + barriers, alignment slack
+  // tap (3 ky + kx) of the lower or upper half of an accumulator
+  static __device__ __forceinline__ int tap(int acc, int half, int kx) {
+    if (G == 3) return acc == 0 ? 3 * half + kx : half == 0 ? 6 + kx : -1;
+    return acc < 3 ? 3 * half + acc : acc == 3 ? 6 + half : half == 0 ? 8 : -1;
+  }
+};
 
+template <int G>
 __global__ void __launch_bounds__(kThreads, 1)
     wgrad_tc_kernel(const __grid_constant__ CUtensorMap dymap,
                     const __grid_constant__ CUtensorMap xmap, WgTcArgs a) {
+  using C = WgCfg<G>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *base = smem_raw + pad;
-  // a stage is filled in two parts: dy and the boxes of kx 0 and 1, then that of kx 2
-  uint64_t *full = reinterpret_cast<uint64_t *>(base + kWgStages * kWgStage);  // [stage][part]
-  uint64_t *empty = full + 2 * kWgStages;
-  uint64_t *done = empty + kWgStages;
+  // a stage is filled in two parts: dy and the boxes of kx 0 and 1 (or of the one kx),
+  // then that of kx 2
+  uint64_t *full = reinterpret_cast<uint64_t *>(base + C::kStages * C::kStage);  // [stage][part]
+  uint64_t *empty = full + 2 * C::kStages;
+  uint64_t *done = empty + C::kStages;
   uint64_t *drain = done + 1;
   uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
   volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // work item: (co tile, ci tile, K split)
+  // work item: (co tile, ci tile, K split, kx where a CTA has one)
   int w = (int)blockIdx.x;
+  const int kx0 = w % G;
+  w /= G;
   const int ks = w % a.ksplit;
   w /= a.ksplit;
   const int cit = w % a.ci_tiles, cot = w / a.ci_tiles;
   const int64_t b0 = a.nblk * ks / a.ksplit, b1 = a.nblk * (ks + 1) / a.ksplit;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2 * kWgStages; s++) mbar_init(&full[s], 1);
-    for (int s = 0; s < kWgStages; s++) mbar_init(&empty[s], 1);
+    for (int s = 0; s < 2 * C::kStages; s++) mbar_init(&full[s], 1);
+    for (int s = 0; s < C::kStages; s++) mbar_init(&empty[s], 1);
     mbar_init(done, 1);
     mbar_init(drain, 1);
     *s_abort = 0;
@@ -1021,7 +1136,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(s_tmem)),
-                 "r"(512u)
+                 "r"(C::kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -1044,10 +1159,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int tx = (int)(blk % a.bx);
         const int64_t r = blk / a.bx;
         const int ty = (int)(r % a.by), b = (int)(r / a.by);
-        uint8_t *sx = base + stage * kWgStage, *sd = sx + 3 * kWgBox;
-        const bool stall = __ldg(&g_test_stall) && blk == b0;
+        uint8_t *sx = base + stage * C::kStage, *sd = sx + C::kBoxes * kWgBox;
+        const bool stall = blk == b0 && __ldg(&g_test_stall);
         auto box = [&](int kx, uint64_t *bar) {
-          tma_load_4d(sx + kx * kWgBox, &xmap, cit * 64, tx * 16 + kx - 1, ty * 8 - 1, b, bar);
+          tma_load_4d(sx + kx * kWgBox, &xmap, cit * 64, tx * 16 + kx0 + kx - 1, ty * 8 - 1, b, bar);
         };
         ok = mbar_wait(&empty[stage], ph ^ 1);
         if (!ok) {
@@ -1055,69 +1170,87 @@ __global__ void __launch_bounds__(kThreads, 1)
           *s_abort = 1;
           break;
         }
-        mbar_expect_tx(&full[2 * stage], (uint32_t)(2 * kWgBox + 8 * kWgRow));
-        mbar_expect_tx(&full[2 * stage + 1], (uint32_t)kWgBox);
+        mbar_expect_tx(&full[2 * stage], (uint32_t)((G == 1 ? 2 : 1) * kWgBox + 8 * kWgRow));
+        if (G == 1) mbar_expect_tx(&full[2 * stage + 1], (uint32_t)kWgBox);
         if (!stall) {
           tma_load_4d(sd, &dymap, cot * 64, tx * 16, ty * 8, b, &full[2 * stage]);
           box(0, &full[2 * stage]);
-          box(1, &full[2 * stage]);
-          box(2, &full[2 * stage + 1]);
+          if (G == 1) {
+            box(1, &full[2 * stage]);
+            box(2, &full[2 * stage + 1]);
+          }
         }
         issued |= 1u << stage;
         last_par = (last_par & ~(1u << stage)) | (ph << stage);
-        if (++stage == kWgStages) {
+        if (++stage == C::kStages) {
           stage = 0;
           ph ^= 1;
         }
       }
-      for (int s = 0; s < kWgStages; s++)
+      for (int s = 0; s < C::kStages; s++)
         if ((issued >> s) & 1u)
-          for (int part = 0; part < 2; part++)
+          for (int part = 0; part < (G == 1 ? 2 : 1); part++)
             if (!mbar_wait(&full[2 * s + part], (last_par >> s) & 1u)) atomicOr(a.err, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------ MMA issuer
+    {
+      // ------------------------------------------------ MMA issuer (whole warp)
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                              ((uint32_t)(a.n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       int stage = 0;
       uint32_t ph = 0, more = 0;
-      for (int64_t blk = b0; blk < b1 && !*s_abort; blk++) {
-        const uint32_t sx = smem_u32(base + stage * kWgStage);
-        const uint64_t db = sdesc_mn128(sx + 3 * kWgBox, kWgRow);
-        // accumulator acc over the block's eight pixel rows
-        auto rows = [&](int acc, uint64_t da) {
-#pragma unroll
-          for (int k = 0; k < 8; k++)
-            tc_mma(tmem + (uint32_t)(64 * acc), da + (uint64_t)(k * (kWgRow >> 4)),
-                   db + (uint64_t)(k * (kWgRow >> 4)), idesc, more | (uint32_t)k);
+      for (int64_t blk = b0; blk < b1 && !__shfl_sync(0xffffffffu, *s_abort, 0); blk++) {
+        const uint32_t sx = smem_u32(base + stage * C::kStage);
+        const uint64_t db = sdesc_mn128(sx + C::kBoxes * kWgBox, kWgRow);
+        auto row = [&](int acc, int k, uint64_t da) {  // pixel row k of the block
+          tc_mma_w(tmem + (uint32_t)(64 * acc), da + (uint64_t)(k * (kWgRow >> 4)),
+                 db + (uint64_t)(k * (kWgRow >> 4)), idesc, more | (uint32_t)k);
         };
-        bool ok = mbar_wait(&full[2 * stage], ph);
+        bool ok = __all_sync(0xffffffffu, mbar_wait(&full[2 * stage], ph));
         if (ok) {
           tc_fence_after();
-          rows(0, sdesc_mn128(sx, kWgRow));                       // ky 0, 1 of kx 0
-          rows(1, sdesc_mn128(sx + kWgBox, kWgRow));              // ky 0, 1 of kx 1
-          rows(3, sdesc_mn128(sx + 2 * kWgRow, kWgBox));          // ky 2 of kx 0, 1
-          ok = mbar_wait(&full[2 * stage + 1], ph);
+          if constexpr (G == 3) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              row(0, k, sdesc_mn128(sx, kWgRow));                 // ky 0, 1
+              row(1, k, sdesc_mn128(sx + 2 * kWgRow, kWgRow));    // ky 2 (lower half)
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              row(0, k, sdesc_mn128(sx, kWgRow));                 // ky 0, 1 of kx 0
+              row(1, k, sdesc_mn128(sx + kWgBox, kWgRow));        // ky 0, 1 of kx 1
+              row(3, k, sdesc_mn128(sx + 2 * kWgRow, kWgBox));    // ky 2 of kx 0, 1
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[2 * stage + 1], ph));
+          }
         }
         if (!ok) {
-          atomicOr(a.err, 1);
-          *s_abort = 1;
+          if (lane == 0) {
+            atomicOr(a.err, 1);
+            *s_abort = 1;
+          }
           break;
         }
         tc_fence_after();
-        rows(2, sdesc_mn128(sx + 2 * kWgBox, kWgRow));            // ky 0, 1 of kx 2
-        // ky 2 of kx 2; the upper half (the rows below, or dy's first) is not used
-        rows(4, sdesc_mn128(sx + 2 * kWgBox + 2 * kWgRow, kWgRow));
-        tc_commit(&empty[stage]);
+        // ky 0, 1 of kx 2; ky 2 of kx 2, whose upper half (the rows below, or dy's
+        // first) is not used
+        if constexpr (G == 1) {
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
+            row(2, k, sdesc_mn128(sx + 2 * kWgBox, kWgRow));
+            row(4, k, sdesc_mn128(sx + 2 * kWgBox + 2 * kWgRow, kWgRow));
+          }
+        }
+        tc_commit_w(&empty[stage]);
         more = 1;
-        if (++stage == kWgStages) {
+        if (++stage == C::kStages) {
           stage = 0;
           ph ^= 1;
         }
       }
-      tc_commit(done);
-      tc_commit(drain);
+      tc_commit_w(done);
+      tc_commit_w(drain);
       if (!mbar_wait(drain, 0)) atomicOr(a.err, 1);
     }
   } else {
@@ -1134,8 +1267,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       // channels
       const int half = row >> 6, ci = cit * 64 + (row & 63);
 #pragma unroll 1
-      for (int acc = 0; acc < kWgAcc; acc++) {
-        const int tap = wg_tap(acc, half);
+      for (int acc = 0; acc < C::kAcc; acc++) {
+        const int tap = C::tap(acc, half, kx0);
 #pragma unroll 1
         for (int c0 = 0; c0 < a.n; c0 += 16) {
           uint32_t rr[16];
@@ -1157,7 +1290,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::kCols)
                  : "memory");
 }
 
@@ -1175,6 +1308,17 @@ bool make_nhwc_map(const __nv_bfloat16 *p, int cs, int co, int C, int W, int H, 
              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
          CUDA_SUCCESS;
+}
+
+template <int G>
+cudaError_t launch_wgrad(const CUtensorMap &dymap, const CUtensorMap &xmap, const WgTcArgs &w,
+                         int tiles, cudaStream_t st) {
+  constexpr int smem = WgCfg<G>::kSmem;
+  const cudaError_t e =
+      cudaFuncSetAttribute(wgrad_tc_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  wgrad_tc_kernel<G><<<(unsigned)(tiles * w.ksplit * G), kThreads, smem, st>>>(dymap, xmap, w);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -1200,12 +1344,9 @@ bool conv_row_ok(const ConvArgs &a) {
 
 cudaError_t launch_conv3x3_row(const ConvArgs &a, cudaStream_t st) {
   if (!conv_row_ok(a)) return cudaErrorInvalidValue;
-  CUtensorMap amap;
-  if (!make_row_map(a, &amap)) return cudaErrorInvalidValue;
+  CUtensorMap amap, ymap;
+  if (!make_row_map(a, &amap) || !make_out_map(a, 32, 1, &ymap)) return cudaErrorInvalidValue;
   RowArgs r{};
-  r.y = a.y;
-  r.y_cs = a.y_cs;
-  r.y_co = a.y_co;
   r.mask = a.mask;
   r.m_cs = a.m_cs;
   r.m_co = a.m_co;
@@ -1216,12 +1357,15 @@ cudaError_t launch_conv3x3_row(const ConvArgs &a, cudaStream_t st) {
   r.relu = a.relu;
   r.H = a.H;
   r.W = a.W;
-  r.nacc = 256 / a.cout >= 8 ? 8 : 256 / a.cout >= 4 ? 4 : 2;
-  r.cols = 256u;
+  // half of tensor memory for each of two CTAs per SM, all of it for one
+  r.cols = row_smem(a, 4) <= kRowSmemHalf ? 256u : 512u;
+  r.nacc = std::min<int>(kMaxAcc, (int)r.cols / a.cout);
   r.wbytes = row_wbytes(a);
   r.slot_bytes = ((a.cin + 63) / 64) * kRowChunkBytes;
+  // two CTAs per SM where four input rows fit beside the weights, else one
+  const int most = r.cols == 256u ? kRowSmemHalf : kRowSmemMax;
   int slots = kRowMaxSlots;
-  while (slots > 4 && row_smem(a, slots) > 110 * 1024) slots--;  // two CTAs per SM if possible
+  while (slots > 4 && row_smem(a, slots) > most) slots--;
   r.nslots = slots;
   cudaError_t e = err_word(&r.err);
   if (e != cudaSuccess) return e;
@@ -1247,7 +1391,7 @@ cudaError_t launch_conv3x3_row(const ConvArgs &a, cudaStream_t st) {
   r.strips_y = (a.H + sh - 1) / sh;
   r.total = (int64_t)a.B * r.strips_y * r.strips_x;
   const int64_t grid = std::min<int64_t>(r.total, ctas);
-  kern<<<(unsigned)grid, kThreads, smem, st>>>(amap, r);
+  kern<<<(unsigned)grid, kThreads, smem, st>>>(amap, ymap, r);
   return cudaGetLastError();
 }
 
@@ -1289,13 +1433,17 @@ cudaError_t launch_conv3x3_wgrad_tc(const WgradArgs &a, cudaStream_t st) {
   w.n = std::min(64, a.cout);
   w.ci_tiles = (a.cin + 63) / 64;
   const int tiles = w.ci_tiles * ((a.cout + 63) / 64);
-  w.ksplit = (int)std::max<int64_t>(1, std::min<int64_t>(w.nblk, sm_count() / tiles));
+  // K splits: as many as fill the device twice with tiles of 128 output channels x 64 or
+  // 128 input channels x one tap.  The tensor cores' accumulation truncates, so the
+  // split decides the result to 1e-4 of it, and stays where it was when a CTA had one
+  // such tile.
+  const int64_t cols = 9LL * ((a.cout + 127) / 128) * (a.cin > 64 ? (a.cin + 127) / 128 : 1);
+  w.ksplit = (int)std::max<int64_t>(1, std::min<int64_t>(w.nblk, (2LL * sm_count() + cols - 1) / cols));
   cudaError_t e = err_word(&w.err);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
-  if (e != cudaSuccess) return e;
-  wgrad_tc_kernel<<<(unsigned)(tiles * w.ksplit), kThreads, kWgSmem, st>>>(dymap, xmap, w);
-  return cudaGetLastError();
+  // a CTA per kx where the nine-tap CTAs would leave most of the device idle
+  return 2 * tiles * w.ksplit <= sm_count() ? launch_wgrad<3>(dymap, xmap, w, tiles, st)
+                                            : launch_wgrad<1>(dymap, xmap, w, tiles, st);
 }
 
 int conv_tc_error() {
