@@ -46,6 +46,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/ctas_learned.h"
 #include "../../include/ctas_fbp.h"
@@ -888,23 +889,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t R = (uint32_t)a.nacc;
       const uint32_t wrow = (uint32_t)cout * row16;  // one block of cout weight rows
       const uint32_t kxblk = 3u * wrow;               // one (kx, chunk) weight block
-      // Ring segments of the output-row counters o .. o + nb - 1 (weight rows
-      // from block position p), split where the ring wraps: TMEM column,
-      // instruction descriptor (N) and weight offset of each, computed once per
-      // input row so that the MMA loop below only adds constant offsets
-      struct Seg {
-        uint32_t d, idesc;
-        uint64_t boff;
-      };
-      auto segments = [&](uint32_t o, uint32_t nb, uint32_t p, Seg *sg) -> int {
-        const uint32_t g = o % R, n1 = min(nb, R - g);
-        sg[0] = Seg{tmem + g * (uint32_t)cout, idesc0 | (((n1 * (uint32_t)cout) >> 3) << 17),
-                    (uint64_t)(p * wrow)};
-        if (n1 == nb) return 1;
-        sg[1] = Seg{tmem, idesc0 | ((((nb - n1) * (uint32_t)cout) >> 3) << 17),
-                    (uint64_t)((p + n1) * wrow)};
-        return 2;
-      };
+      // instruction descriptor of n output-row blocks
+      auto idesc_n = [&](uint32_t n) { return idesc0 | (((n * (uint32_t)cout) >> 3) << 17); };
       uint32_t j0 = 0, o0 = 0;
       bool ok = true;
       for (int64_t t = blockIdx.x; t < a.total && ok && !__shfl_sync(0xffffffffu, *s_abort, 0);
@@ -929,36 +915,40 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           tc_fence_after();
           const uint64_t da = sdesc_sw128(slots_u + (jl % (uint32_t)ns) * (uint32_t)a.slot_bytes);
+          // blocks of the rows lo..hi (weight rows from block position p0), split in two
+          // where the ring wraps: TMEM column, N and weight offset of both parts as
+          // plain scalars, so that the MMAs below take them from uniform registers
           const uint32_t nb = (uint32_t)(hi - lo + 1), p0 = (uint32_t)(lo - yi + 1);
-          // all rows lo..hi (accumulating), and for the first MMA of a fresh
-          // row yi + 1: rows lo..hi - 1 accumulating, row hi overwritten
-          Seg all[2], head[3];
-          const int nall = segments(olo, nb, p0, all);
-          int nhead = 0, nacc_head = 0;
+          const uint32_t g = olo % R, n0 = min(nb, R - g), n1 = nb - n0;
+          const uint32_t d0 = tmem + g * (uint32_t)cout, i0 = idesc_n(n0), i1 = idesc_n(n1);
+          const uint64_t w0 = dw0 + (uint64_t)(p0 * wrow), w1 = dw0 + (uint64_t)((p0 + n0) * wrow);
           if (fresh) {
-            if (nb > 1) nhead = segments(olo, nb - 1, p0, head);
-            nacc_head = nhead;
-            nhead += segments(ohi, 1, p0 + nb - 1, head + nhead);
+            // the first MMA of row yi + 1: rows lo..hi - 1 accumulate, row hi starts
+            const uint32_t h0 = min(nb - 1u, n0), h1 = nb - 1u - h0;
+            if (h0) tc_mma_w(d0, da, w0, idesc_n(h0), 1u);
+            if (h1) tc_mma_w(tmem, da, w1, idesc_n(h1), 1u);
+            tc_mma_w(tmem + (ohi % R) * (uint32_t)cout, da, dw0 + (uint64_t)((p0 + nb - 1u) * wrow),
+                     idesc_n(1u), 0u);
+          } else {
+            tc_mma_w(d0, da, w0, i0, 1u);
+            if (n1) tc_mma_w(tmem, da, w1, i1, 1u);
           }
+          auto rest = [&](auto two) {
 #pragma unroll
-          for (int kx = 0; kx < 3; kx++)
-#pragma unroll
-            for (int st = 0; st < cin / 16; st++) {
-              // 16-channel step st: row chunk st / 4, 32-byte column st % 4;
+            for (int q = 1; q < 3 * (cin / 16); q++) {
+              // 16-channel step st of kx: row chunk st / 4, 32-byte column st % 4;
               // weights: block (kx, st / kSteps), 32-byte column st % kSteps
+              const int kx = q / (cin / 16), st = q % (cin / 16);
               const uint64_t a_op =
                   da + (uint64_t)(((st >> 2) * kRowChunkBytes + kx * 128 + (st & 3) * 32) >> 4);
-              const uint64_t b_op =
-                  dw0 + (uint64_t)((uint32_t)(kx * kChunks + st / kSteps) * kxblk +
-                                   (uint32_t)((st % kSteps) * 2));
-              if (kx == 0 && st == 0 && fresh) {
-                for (int q = 0; q < nhead; q++)
-                  tc_mma_w(head[q].d, a_op, b_op + head[q].boff, head[q].idesc, q < nacc_head ? 1u : 0u);
-              } else {
-                tc_mma_w(all[0].d, a_op, b_op + all[0].boff, all[0].idesc, 1u);
-                if (nall > 1) tc_mma_w(all[1].d, a_op, b_op + all[1].boff, all[1].idesc, 1u);
-              }
+              const uint64_t b_off = (uint64_t)((uint32_t)(kx * kChunks + st / kSteps) * kxblk +
+                                                (uint32_t)((st % kSteps) * 2));
+              tc_mma_w(d0, a_op, w0 + b_off, i0, 1u);
+              if constexpr (decltype(two)::value) tc_mma_w(tmem, a_op, w1 + b_off, i1, 1u);
             }
+          };
+          if (n1) rest(std::true_type{});
+          else rest(std::false_type{});
           tc_commit_w(&row_empty[jl % (uint32_t)ns]);       // input row yi is done
           if (yi - 1 >= r0) tc_commit_w(&acc_full[olo % R]);  // output row yi - 1 is complete
         }
