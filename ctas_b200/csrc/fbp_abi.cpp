@@ -250,10 +250,14 @@ bool quad_capable(const ctas_fbp *h) {
 
 // How many of S slices (the first ones) go through the four-slice kernel: whole
 // groups, and a group of the last three.  One or two slices left over take the
-// one-slice kernel: a group's time is that of 2.2 slices of 1800 x 2560 alone.
+// one-slice kernel (a group's time is that of 2.2 slices of 1800 x 2560 alone), unless
+// they are so small that a launch of their own leaves most of the device idle: the last
+// slice of 29 of 1784 x 296 takes 230 us alone and 115 us as a group more.
 int64_t quad_count(const ctas_fbp *h, int64_t S) {
   if (S < 3 || !quad_capable(h)) return 0;
-  const int64_t rest = S % ctas::kQuadSlices, n = rest == 3 ? S : S - rest;
+  const int64_t rest = S % ctas::kQuadSlices;
+  const bool small = ((h->out_rows + 63) / 64) * ((h->out_cols + 63) / 64) <= 48;
+  const int64_t n = rest == 3 || small ? S : S - rest;
   if (!(h->flags & CTAS_FLAG_GROUPS) && !ctas::bp_quad_pays(h->out_rows, h->out_cols, n, h->sms))
     return 0;
   return n;
