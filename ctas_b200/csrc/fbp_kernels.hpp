@@ -63,6 +63,7 @@ struct FilterLaunch {
                              // element p < 2W = sample (p - zs) mod W, 0 beyond;
                              // with a window symmetric about 0 this is the row's
                              // circular convolution of length W (unpadded filter)
+  float dc;                  // periodic: the filter's response to a row of ones
   int off;                   // column of sample 0 in the output rows; 0 = kRowOff
   int quad;                  // 1: interleaved layout (float32; q_slice_stride is then a
                              // group's, in floats)

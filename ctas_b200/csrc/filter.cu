@@ -48,6 +48,14 @@ template <int R>
 __device__ __forceinline__ void twiddles(const float4 *__restrict__ tws, int m, float2 *w) {
   const float4 e = __ldg(&tws[m]);
   w[1] = make_float2(e.x, e.y);
+  if (R == 3 || R == 5) {  // the entry is (w, w^2)
+    w[2] = make_float2(e.z, e.w);
+    if (R == 5) {
+      w[3] = cmul(w[2], w[1]);
+      w[4] = cmul(w[2], w[2]);
+    }
+    return;
+  }
   if (R >= 4) {
     w[2] = cmul(w[1], w[1]);
     w[3] = cmul(w[2], w[1]);
@@ -101,8 +109,35 @@ template <int DIR> __device__ __forceinline__ void dft8(float2 *x) {
   x[3] = e[3] + w3;
   x[7] = e[3] - w3;
 }
+template <int DIR> __device__ __forceinline__ void dft3(float2 *x) {
+  const float s = 0.86602540378443864676f;  // sin 60
+  const float2 t = x[1] + x[2], d = x[1] - x[2];
+  const float2 a = make_float2(x[0].x - 0.5f * t.x, x[0].y - 0.5f * t.y);
+  const float2 b = mul_i<DIR>(make_float2(s * d.x, s * d.y));
+  x[0] = x[0] + t;
+  x[1] = a + b;
+  x[2] = a - b;
+}
+template <int DIR> __device__ __forceinline__ void dft5(float2 *x) {
+  // cos 72, 144 = (-1 +- sqrt 5) / 4: in this form a constant row gives exact zeros
+  const float r = 0.55901699437494742410f;  // sqrt 5 / 4
+  const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;  // sin 72, 144
+  const float2 t1 = x[1] + x[4], t2 = x[2] + x[3], d1 = x[1] - x[4], d2 = x[2] - x[3];
+  const float2 t = t1 + t2, a = make_float2(x[0].x - 0.25f * t.x, x[0].y - 0.25f * t.y);
+  const float2 e = make_float2(r * (t1.x - t2.x), r * (t1.y - t2.y));
+  const float2 a1 = a + e, a2 = a - e;
+  const float2 b1 = mul_i<DIR>(make_float2(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y));
+  const float2 b2 = mul_i<DIR>(make_float2(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y));
+  x[0] = x[0] + t;
+  x[1] = a1 + b1;
+  x[4] = a1 - b1;
+  x[2] = a2 + b2;
+  x[3] = a2 - b2;
+}
 template <int R, int DIR> __device__ __forceinline__ void dft(float2 *x) {
   if (R == 2) dft2<DIR>(x);
+  if (R == 3) dft3<DIR>(x);
+  if (R == 5) dft5<DIR>(x);
   if (R == 4) dft4<DIR>(x);
   if (R == 8) dft8<DIR>(x);
 }
@@ -269,8 +304,9 @@ __device__ __forceinline__ float pow2_scale(float mx) {
 }
 
 // Filters rows 2*pair and 2*pair+1 of slice sl.  Called by every thread of
-// the CTA with the CTA's dynamic shared memory (P + P/32 float2).
-template <typename T>
+// the CTA with the CTA's dynamic shared memory (P + P/16 float2).  ODD: P is 3 or 5
+// times a power of two, its first radix 3 or 5 (every later stride is a power of two).
+template <typename T, bool ODD = false>
 __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int sl) {
   extern __shared__ float2 sm[];
   __shared__ float red[2][kFftThreads / 32];
@@ -292,6 +328,34 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
     if (r1 + 1 < N) qb = deabs(qb, mm);
   }
 
+  // Periodic rows of odd plans are transformed less their mean, and the response to that
+  // constant is added back.  They fill the transform (two periods in 2n elements or
+  // little more), whose rounding is relative to what it holds: without this its error is
+  // 15 to 28 % above that of the next power of two.
+  float2 mean = make_float2(0.f, 0.f);
+  if (ODD && a.periodic) {
+    // one sample a thread, evenly spaced, is mean enough (all of them cost 17 % more)
+    const int c = threadIdx.x * W / (int)blockDim.x;
+    mean.x = abs_mode ? deabs(x0[c], mm) : x0[c];
+    if (has1) mean.y = abs_mode ? deabs(x1[c], mm) : x1[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      mean.x += __shfl_xor_sync(0xffffffffu, mean.x, o);
+      mean.y += __shfl_xor_sync(0xffffffffu, mean.y, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      red[0][threadIdx.x >> 5] = mean.x;
+      red[1][threadIdx.x >> 5] = mean.y;
+    }
+    __syncthreads();
+    mean = make_float2(0.f, 0.f);
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) mean = mean + make_float2(red[0][w], red[1][w]);
+    mean = make_float2(mean.x / (float)blockDim.x, mean.y / (float)blockDim.x);
+  }
+  auto with_mean = [&](float2 z) {
+    return ODD && a.periodic ? make_float2(z.x + mean.x * a.dc, z.y + mean.y * a.dc) : z;
+  };
+
   // element p of the zero-padded row pair
   auto load = [&](int p) -> float2 {
     int c = p - zs;
@@ -308,6 +372,7 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
         v.x = deabs(v.x, mm);
         if (has1) v.y = deabs(v.y, mm);
       }
+      if (ODD && a.periodic) v = v - mean;
     } else if (c == W && !a.periodic) {
       v = make_float2(qa, qb);
     }
@@ -342,7 +407,9 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
 
   if (ns >= 2) {
     const int R = a.radix[0];
-    if (R == 8) dif_first_stage<8>(sm, hs[0], tws, load);
+    if (ODD && R == 5) dif_first_stage<5>(sm, hs[0], tws, load);
+    else if (ODD) dif_first_stage<3>(sm, hs[0], tws, load);
+    else if (R == 8) dif_first_stage<8>(sm, hs[0], tws, load);
     else if (R == 4) dif_first_stage<4>(sm, hs[0], tws, load);
     else dif_first_stage<2>(sm, hs[0], tws, load);
   } else {
@@ -361,13 +428,20 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
   }
   __syncthreads();
   for (int st = ns - 2; st >= (direct ? 1 : 0); st--) {
-    run_stage<false>(sm, P, a.radix[st], hs[st], tws + to[st]);
+    if (ODD && st == 0) {  // in place: every thread writes the elements that it read
+      auto keep = [&](int p, float2 v) { sm[sidx(p)] = with_mean(v); };
+      if (a.radix[0] == 5) dit_last_stage<5>(sm, hs[0], tws, keep);
+      else dit_last_stage<3>(sm, hs[0], tws, keep);
+    } else {
+      run_stage<false>(sm, P, a.radix[st], hs[st], tws + to[st]);
+    }
     __syncthreads();
   }
   if (direct) {
     auto store = [&](int p, float2 z) {
       const int c = p - zs;
       if (c < 0 || c >= W) return;
+      z = with_mean(z);
       q0[c * es] = to_store<T>(z.x);
       if (has1) q1[c * es] = to_store<T>(z.y);
       if (d0) {
@@ -389,7 +463,9 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
       }
     };
     const int R = a.radix[0];
-    if (R == 8) dit_last_stage<8>(sm, hs[0], tws, store);
+    if (ODD && R == 5) dit_last_stage<5>(sm, hs[0], tws, store);
+    else if (ODD) dit_last_stage<3>(sm, hs[0], tws, store);
+    else if (R == 8) dit_last_stage<8>(sm, hs[0], tws, store);
     else if (R == 4) dit_last_stage<4>(sm, hs[0], tws, store);
     else dit_last_stage<2>(sm, hs[0], tws, store);
     return;
@@ -493,6 +569,10 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
 template <typename T>
 __global__ void __launch_bounds__(kFftThreads) filter_rows_kernel(FilterLaunch a) {
   filter_pair<T>(a, blockIdx.x, blockIdx.y);
+}
+
+__global__ void __launch_bounds__(kFftThreads) filter_odd_kernel(FilterLaunch a) {
+  filter_pair<float, true>(a, blockIdx.x, blockIdx.y);
 }
 
 // Interleaved layout: the four slices of a group write the same 32-byte sectors, so
@@ -713,6 +793,16 @@ cudaError_t launch_filter_t(const FilterLaunch &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+cudaError_t launch_filter_odd(const FilterLaunch &a, cudaStream_t st) {
+  if (a.store != 0 || a.quad || a.nradix < 2) return cudaErrorInvalidValue;
+  const size_t smem = sizeof(float2) * (size_t)(a.P + a.P / 16);
+  const cudaError_t e = cudaFuncSetAttribute(
+      filter_odd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  filter_odd_kernel<<<dim3((a.N + 1) / 2, a.S), kFftThreads, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_filter_quad(const FilterLaunch &a, cudaStream_t st) {
   const size_t smem = sizeof(float2) * (size_t)(a.P + a.P / 16);
   if (smem > 48 * 1024) {
@@ -764,6 +854,8 @@ cudaError_t launch_expand_quad(const void *q, int64_t q_slice_stride, const floa
 }
 
 cudaError_t launch_filter(const FilterLaunch &a, cudaStream_t st) {
+  if (a.contrast != 3 && a.nradix > 0 && (a.radix[0] == 3 || a.radix[0] == 5))
+    return launch_filter_odd(a, st);
   if (a.quad && a.store != 0) return cudaErrorInvalidValue;
   if (a.quad && a.contrast != 3) return launch_filter_quad(a, st);
   if (a.store == 1) return launch_filter_t<__half>(a, st);

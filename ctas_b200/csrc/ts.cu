@@ -4,13 +4,14 @@
 //
 // Filter.  The reference filters each row of length n (= pixels) with
 // HC2R(R2HC(z) * f) / n, f = Filter::fill(n): a circular convolution of length
-// n with the real, even kernel g = IDFT_n(f).  The device FFT is a power of two
-// P >= 2n - 1 (the CT padding rule), so the row is extended periodically (two
-// periods from offset n/2; filter kernel "periodic" mode) and multiplied by
-// G_P = DFT_P(h), h the kernel g laid out symmetrically about 0 (|d| <= n/2;
-// for even n the d = n/2 tap is split between +-n/2).  For outputs n/2 ..
-// 3n/2 - 1 every tap reads inside the two periods, so the result is the
-// circular convolution up to float rounding.
+// n with the real, even kernel g = IDFT_n(f).  The device FFT has a length P >= 2n,
+// so the row is extended periodically (two periods from offset n/2; filter kernel
+// "periodic" mode) and multiplied by G_P = DFT_P(h), h the kernel g laid symmetrically
+// about 0 (|d| <= n/2; for even n the d = n/2 tap is split between +-n/2).  For outputs
+// n/2 .. 3n/2 - 1 every tap reads inside the two periods, so the result is the circular
+// convolution up to float rounding.  P is the least of 2^k, 3 2^k and 5 2^k: the filter
+// is bound by its passes over P elements in shared memory (5120 instead of 8192 for
+// rows of 2560).
 //
 // Backprojection.  One thread per result pixel adds the n images' terms in
 // order, with the reference's float expression for the sample index.
@@ -117,6 +118,7 @@ struct ctas_ts {
   int device = 0;
   int64_t rows = 0, W = 0, P = 0, Wp = 0;
   int32_t contrast = 2;
+  float dc = 0.f;  // response of the filter to a row of ones
   std::vector<int> radices;
   cudaStream_t stream = nullptr;  // host calls
   Buf tw, gperm, q, cs, host_in, host_out;
@@ -184,17 +186,23 @@ void ts_create(ctas_ts *h, int64_t rows, int64_t pixels, int32_t ftype, float fp
   h->P = ctas::padded_width(pixels);
   if (h->P > 16384)  // the row-pair FFT lives in shared memory
     ctas::fail(CTAS_E_UNSUPPORTED, "tomosynthesis: rows wider than 8192 pixels are not supported");
+  for (const int64_t odd : {3, 5}) {
+    int64_t P = 16 * odd;
+    while (P < 2 * pixels) P *= 2;
+    h->P = std::min(h->P, P);
+  }
   h->Wp = ctas::padded_pitch(pixels);
   // ts_add filters for every contrast; ABS adds -log, REF the running sum
   h->contrast = contrast == CTAS_FLT ? CTAS_PHS : contrast;
   h->radices = ctas::fft_radices(h->P);
   const std::vector<float> fwin = ctas::filter_fill(ftype, fparam, pixels);  // Filter::fill(n)
+  h->dc = fwin[0];
   const std::vector<double> G = ts_window(fwin, pixels, h->P);
   const auto perm = ctas::fft_output_order(h->P, h->radices);
   std::vector<float> gp((size_t)h->P);
-  const float invP = 1.0f / (float)h->P;
-  for (int64_t p = 0; p < h->P; p++) gp[(size_t)p] = (float)G[(size_t)perm[(size_t)p]] * invP;
-  const auto tw = ctas::fft_twiddles(h->P);
+  for (int64_t p = 0; p < h->P; p++)
+    gp[(size_t)p] = (float)(G[(size_t)perm[(size_t)p]] / (double)h->P);
+  const auto tw = ctas::fft_twiddles(h->P, h->radices);
   DevGuard g(dev);
   cuda_check(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
   h->tw.ensure(sizeof(float) * tw.size());
@@ -247,6 +255,7 @@ void ts_run(ctas_ts *h, float *proj, const float *angles, int64_t n, float *resu
     a.S = (int)m;
     a.guard = 0;
     a.periodic = 1;
+    a.dc = h->dc;
     cuda_check(ctas::launch_filter(a, st), "filter kernel");
     TsBpLaunch b{};
     b.q = h->q.as<float>();
