@@ -242,12 +242,13 @@ def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_pea
               "peak": round(l2_peak_gbs, 1), "frac": round(l2_ach / l2_peak_gbs, 4),
               "unit": "GB/s", "peak_source": "measured in this run by ctas_probe_l2_read "
                                             "(16-byte L2 reads of a 32 MiB buffer)"}
+    groups = tile is not None and tile < 0   # no tile id: the four-slice kernel
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if os.path.exists(tpath):
         with open(tpath) as f:
             tr = json.load(f)
-        if "bp_fast_per_slice_bytes" in tr:
+        if not groups and "bp_fast_per_slice_bytes" in tr:
             traffic = tr["bp_fast_per_slice_bytes"] * slices_per_launch
     filt_bytes = 4.0 * N_ANGLES * WIDTH * 2 * slices_per_launch   # read + write rows
     hbm_peak = 6541.8
@@ -272,7 +273,9 @@ def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_pea
                   "the nominal 128 B/clk/SM; this term, not HBM, bounds the filter"}
     nominal = 128.0 * sms * (clocks.get("sm_mhz") or 1965.0) * 1e6 / 1e9
     return {
-        "bound": "smem", "kernel": "bp_fast (backprojection)", "unit": "GB/s",
+        "bound": "smem", "unit": "GB/s",
+        "kernel": "bp_quad (backprojection, four slices at a time)" if groups
+                  else "bp_fast (backprojection)",
         "achieved": round(achieved, 1), "peak": round(nominal, 1),
         "frac": round(achieved / nominal, 4),
         "peak_source": "nominal shared-memory load bandwidth: 128 B/clk/SM x SMs x the median "
@@ -287,7 +290,9 @@ def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_pea
                           "this kernel (profiles/ncu_traffic.json, per slice, scaled to the "
                           "launch): a committed measurement, not taken in this run",
         "algorithmic_bytes_per_launch": bp_bytes,
-        "unit_note": "4 B per in-mask update (N x in-mask pixels per slice)",
+        "unit_note": "4 B per in-mask update (N x in-mask pixels per slice)" +
+                     ("; a sample may serve several pixels (0.49 loads per pixel), so this "
+                      "bound of one load per update can be exceeded" if groups else ""),
         "filter": {"bound": "hbm", "unit": "GB/s",
                    "achieved": round(f_ach, 1) if f_ach else None, "peak": hbm_peak,
                    "frac": round(f_ach / hbm_peak, 4) if f_ach else None,
