@@ -224,6 +224,14 @@ namespace {
 
 size_t elem_bytes(int store) { return store == 0 ? 4 : 2; }
 
+// Zeroes a small buffer before anything on any stream can use it.  A plain cudaMemset
+// goes to the legacy stream and returns before it has run: kernels on a non-blocking
+// stream do not wait for it.
+void zero_now(void *p, size_t bytes, cudaStream_t st) {
+  cuda_check(cudaMemsetAsync(p, 0, bytes, st), "cudaMemsetAsync");
+  cuda_check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+}
+
 void init_streams(ctas_fbp *h) {
   cuda_check(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
   cuda_check(cudaStreamCreateWithFlags(&h->s_in, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -234,7 +242,7 @@ void init_streams(ctas_fbp *h) {
     cuda_check(cudaEventCreateWithFlags(&w.ev_out, cudaEventDisableTiming), "cudaEventCreate");
   }
   h->err.ensure(sizeof(int));
-  cuda_check(cudaMemset(h->err.p, 0, sizeof(int)), "cudaMemset");
+  zero_now(h->err.p, sizeof(int), h->stream);
   cuda_check(cudaMallocHost((void **)&h->err_host, sizeof(int)), "cudaMallocHost");
   *h->err_host = 0;
 }
@@ -279,8 +287,9 @@ float *quad_rows(const WorkSet &w) {
 }
 
 // Sizes one work set for S slices or fewer.  The padded filtered buffers are zeroed
-// on allocation: their pad columns are never written afterwards.
-void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw) {
+// on allocation: their pad columns are never written afterwards.  st: the stream whose
+// kernels use them next; the zeros are queued there, ahead of the filter's stores.
+void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw, cudaStream_t st) {
   const int64_t N = h->N, W = h->W;
   if (need_raw) w.raw.ensure(sizeof(float) * (size_t)(S * N * W));
   const int64_t n4 = quad_count(h, S);
@@ -292,10 +301,10 @@ void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw) {
   if (n4 > 0) {
     const int64_t words = quad_resident(h, quad_groups(S)) * N * h->Wp + 2 * ctas::kQuadSlack;
     if (w.quad.ensure(sizeof(float) * ctas::kQuadSlices * (size_t)words))
-      cuda_check(cudaMemset(w.quad.p, 0, w.quad.bytes), "cudaMemset");
+      cuda_check(cudaMemsetAsync(w.quad.p, 0, w.quad.bytes, st), "cudaMemsetAsync");
   }
   if (w.filt.ensure(elem_bytes(h->store) * (size_t)(alone * N * h->Wp)))
-    cuda_check(cudaMemset(w.filt.p, 0, w.filt.bytes), "cudaMemset");
+    cuda_check(cudaMemsetAsync(w.filt.p, 0, w.filt.bytes, st), "cudaMemsetAsync");
   if (h->store != 0) w.scale.ensure(sizeof(float) * (size_t)(S * N));
   w.slice.ensure(sizeof(float) * (size_t)(S * h->out_rows * h->out_cols));
   if (h->contrast == CTAS_ABS) {
@@ -557,7 +566,7 @@ int read_err(ctas_fbp *h, cudaStream_t st) {
 // Maps a non-zero device error word to a status (and clears it).
 void raise_err_word(ctas_fbp *h, int w) {
   if (!w) return;
-  cuda_check(cudaMemset(h->err.p, 0, sizeof(int)), "cudaMemset");
+  zero_now(h->err.p, sizeof(int), h->stream);
   if (w & 1) fail_bad_data();
   if (w & 4) ctas::fail(CTAS_E_TIMEOUT, "a device wait timed out in the backprojection kernel");
   if (w & 8) ctas::fail(CTAS_E_CUDA, "backprojection window check failed");
@@ -991,7 +1000,7 @@ int ctas_fbp_sino(ctas_fbp *h, float *sino) {
     if (!sino) ctas::fail(CTAS_E_ARG, "null sinogram");
     DeviceGuard g(h->device);
     WorkSet &w = h->ws[0];
-    ensure_set(h, w, 1, true);
+    ensure_set(h, w, 1, true, h->stream);
     const size_t in_bytes = sizeof(float) * (size_t)(h->N * h->W);
     cuda_check(cudaMemcpyAsync(w.raw.p, sino, in_bytes, cudaMemcpyHostToDevice, h->stream),
                "cudaMemcpyAsync");
@@ -1030,7 +1039,7 @@ int ctas_fbp_reconstruct(ctas_fbp *h, float *sino, float *slice, float center) {
     check_center(h, center);
     DeviceGuard g(h->device);
     WorkSet &w = h->ws[0];
-    ensure_set(h, w, 1, true);
+    ensure_set(h, w, 1, true, h->stream);
     const size_t in_bytes = sizeof(float) * (size_t)(h->N * h->W);
     cuda_check(cudaMemcpyAsync(w.raw.p, sino, in_bytes, cudaMemcpyHostToDevice, h->stream),
                "cudaMemcpyAsync");
@@ -1056,7 +1065,7 @@ int ctas_fbp_sino_dev(ctas_fbp *h, const float *sino_dev, float *filtered_dev, v
     DeviceGuard g(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     WorkSet &w = h->ws[0];
-    ensure_set(h, w, 1, false);
+    ensure_set(h, w, 1, false, st);
     run_filter(h, sino_dev, 1, w, st);
     if (filtered_dev) {
       cuda_check(ctas::launch_unpad(w.filt.p, h->N * h->Wp, h->store ? w.scale.as<float>() : nullptr,
@@ -1112,7 +1121,7 @@ int ctas_fbp_reconstruct_dev(ctas_fbp *h, const float *sino_dev, float *slice_de
     DeviceGuard g(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     WorkSet &w = h->ws[0];
-    ensure_set(h, w, 1, false);
+    ensure_set(h, w, 1, false, st);
     run_filter(h, sino_dev, 1, w, st);
     run_bp(h, w, 1, center, slice_dev, st);
     h->have_sino = true;
@@ -1144,7 +1153,7 @@ int ctas_fbp_reconstruct_stack_dev(ctas_fbp *h, const float *sinos_dev, float *s
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t C = device_chunk(h, n_slices);
     WorkSet &w = h->ws[0];
-    ensure_set(h, w, C, false);
+    ensure_set(h, w, C, false, st);
     for (int64_t s0 = 0; s0 < n_slices; s0 += C) {
       const int64_t S = std::min(C, n_slices - s0);
       run_filter(h, sinos_dev + s0 * h->N * h->W, S, w, st);
@@ -1171,7 +1180,7 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     // stored densely beside them
     const bool dense = wb && h->store == CTAS_STORE_F32 && quad_count(h, C) > 0;
     for (auto &w : h->ws) {
-      ensure_set(h, w, C, true);
+      ensure_set(h, w, C, true, h->stream);
       if (dense) w.dense.ensure(sizeof(float) * (size_t)(C * NW));
     }
     // If a later chunk fails, copies of earlier chunks into the caller's host
@@ -1274,7 +1283,7 @@ int ctas_fbp_reconstruct_volume(ctas_fbp *h, int64_t n_slices, float center, int
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
     const bool own_range = bpp != 0 && mincon == maxcon;
     for (auto &w : h->ws) {
-      ensure_set(h, w, C, true);
+      ensure_set(h, w, C, true, h->stream);
       if (bpp != 0) w.samples.ensure((size_t)(sb * C * OO));
       if (own_range) {
         w.part.ensure(sizeof(float2) * (size_t)(C * ctas::kMinMaxBlocks));
