@@ -842,11 +842,10 @@ bool make_map(const BpLaunch &a, int box, CUtensorMap *map) {
 }
 
 // ------------------------------------------------------------ autotuner
-// Per (device, W, N, store, interp): the tile that ran fastest on this
-// machine.  Candidates are timed on one slice of the caller's own launch, and
-// the winner is cached for the process.
+// Per TuneKey: the tile that ran fastest on this machine.  Candidates are timed on
+// slices of the caller's own launch, and the winner is cached for the process.
 std::mutex g_tune_mutex;
-std::map<std::tuple<int, int, int, int, int, int, int>, int> g_tuned;
+std::map<TuneKey, int> g_tuned;
 
 int env_tile() {
   static const int t = [] {
@@ -966,16 +965,21 @@ int bp_fast_search(const std::function<float(int)> &time_ms, bool all_variants) 
 
 bool bp_fast_tile_forced() { return env_tile() >= 0 && env_tile() < kTiles; }
 
-int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested) {
+int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested, bool rest) {
   if (requested >= 0 && requested < kTiles) return requested;
   if (env_tile() >= 0 && env_tile() < kTiles) return env_tile();
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto key = std::make_tuple(dev, a.W, a.N, a.store, a.interp, a.out_rows, a.out_cols);
+  const TuneKey key = bp_fast_tune_key(a, dev, rest);
   {
     std::lock_guard<std::mutex> g(g_tune_mutex);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) return it->second;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return kShapes * (kVariants - 1) + 1;
   }
   // time the candidates on a few slices of this launch (their output is
   // overwritten by the real launch that follows): enough for about eight

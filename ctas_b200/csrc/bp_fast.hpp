@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <functional>
+#include <tuple>
 
 #include "fbp_kernels.hpp"
 
@@ -20,11 +21,22 @@ const char *bp_fast_error_detail();
 // runs one candidate and returns its time, < 0 if it failed; each candidate
 // runs twice and the second time counts.  Returns -1 if every one failed.
 int bp_fast_search(const std::function<float(int)> &time_ms, bool all_variants);
+// Launches that share the autotuner's choice: one device, geometry and kernel form.
+// The wide layout has kernels of its own, and the one or two slices that a stack
+// leaves over (rest) fill too little of the device to decide for full launches: on
+// nine slices of 1800 x 2560 the tile that two wide slices prefer (14) takes 14.8 ms,
+// the full launch's own (15) 14.2.
+using TuneKey = std::tuple<int, int, int, int, int, int, int, bool, bool>;
+inline TuneKey bp_fast_tune_key(const BpLaunch &a, int device, bool rest) {
+  return TuneKey(device, a.W, a.N, a.store, a.interp, a.out_rows, a.out_cols, a.wide != 0, rest);
+}
 // Tile for this launch: `requested` if it is a valid id, else the
-// CTAS_FBP_TILE environment override, else the autotuner's choice for
-// (device, W, N, store, interp) -- the first launch of a shape runs
-// bp_fast_search on one slice of that launch (synchronising the stream).
-int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested);
+// CTAS_FBP_TILE environment override, else the autotuner's choice for the launch's
+// TuneKey -- the first such launch runs bp_fast_search on a few of its slices
+// (synchronising the stream).  While the stream is being captured nothing can be
+// timed: a launch of a new key then takes the usually fastest tile, which is not kept.
+// rest: the launch is what a stack's four-slice groups leave over.
+int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested, bool rest = false);
 // True when CTAS_FBP_TILE names a tile.
 bool bp_fast_tile_forced();
 cudaError_t launch_bp_fast(const BpLaunch &a, cudaStream_t st, int tile);

@@ -506,8 +506,8 @@ void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, 
                     (h->interp == CTAS_INTERP_LINEAR || h->sines_nonneg || h->wide);
   int tile = -1;
   if (fast)  // may time the tiles once (not for the stalling test aid)
-    tile = ctas::bp_fast_choose_tile(b, st, (h->flags & CTAS_FLAG_TEST_TIMEOUT) && h->tile < 0
-                                                ? 1 : h->tile);
+    tile = ctas::bp_fast_choose_tile(
+        b, st, (h->flags & CTAS_FLAG_TEST_TIMEOUT) && h->tile < 0 ? 1 : h->tile, n4 > 0);
   KernelTimer tm(h, CTAS_KERNEL_BACKPROJECT, st);
   if (fast) {
     const cudaError_t e = (h->flags & CTAS_FLAG_CHECKED) ? ctas::launch_bp_fast_checked(b, st, tile)
