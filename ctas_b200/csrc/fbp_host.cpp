@@ -281,29 +281,28 @@ std::vector<float> fft_twiddles(int64_t P) {
 }
 
 std::vector<float> fft_twiddles(int64_t P, const std::vector<int> &radices) {
-  std::vector<float> tw((size_t)(2 * P), 0.0f);
-  int64_t h = P, off = 0;
+  std::vector<float> tw;
+  int64_t h = P;
   for (const int R : radices) {
     h /= R;
     const int64_t t = P / (R * h);
-    for (int64_t m = 0; m < h; m++)
-      for (int q = 0; q < 2; q++) {
-        const double a = -2.0 * M_PI * (double)(((q ? (R % 2 ? 2 : 4) : 1) * m * t) % P) / (double)P;
-        tw[(size_t)(4 * (off + m) + 2 * q)] = (float)std::cos(a);
-        tw[(size_t)(4 * (off + m) + 2 * q + 1)] = (float)std::sin(a);
-      }
-    off += h;
+    for (int j = 0; j < R / 2; j++)
+      for (int64_t m = 0; m < h; m++)
+        for (int q = 2 * j + 1; q <= 2 * j + 2; q++) {
+          const double a = -2.0 * M_PI * (double)((q * m * t) % P) / (double)P;
+          tw.push_back((float)std::cos(a));
+          tw.push_back((float)std::sin(a));
+        }
   }
   return tw;
 }
 
 std::vector<int> fft_radices(int64_t P) {
-  for (const int odd : {3, 5})
-    if (P % odd == 0) {
-      std::vector<int> r = fft_radices(P / odd);
-      r.insert(r.begin(), odd);
-      return r;
-    }
+  if (P % 3 == 0) {
+    std::vector<int> r = fft_radices(P / 3);
+    r.insert(r.begin(), 3);
+    return r;
+  }
   int lg = 0;
   while ((int64_t(1) << lg) < P) lg++;
   std::vector<int> r;

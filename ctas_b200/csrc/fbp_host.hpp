@@ -43,10 +43,11 @@ float rec_cof(float pixel_size, float lambda);         // lct.cpp:558-566
 // (w^(m t), w^(4 m t)) for each butterfly index m, w = e^{-2 pi i / P},
 // computed in double and rounded.
 std::vector<float> fft_twiddles(int64_t P);
-// the same for any plan; (w^(m t), w^(2 m t)) for a radix of 3 or 5
+// All powers, for a plan with a radix of 3: per stage, for j < R / 2, h_s entries of
+// four floats, (w^((2 j + 1) m t), w^((2 j + 2) m t)), each rounded once.
 std::vector<float> fft_twiddles(int64_t P, const std::vector<int> &radices);
 // Radix plan of the device FFT: stage radices from the largest block down.
-// 8, ..., 8 and a last 2 or 4; first 3 or 5 where P is that times a power of two
+// 8, ..., 8 and a last 2 or 4; first 3 where P is that times a power of two
 std::vector<int> fft_radices(int64_t P);
 // Position p of the device FFT's forward output holds frequency perm[p].
 std::vector<int64_t> fft_output_order(int64_t P, const std::vector<int> &radices);

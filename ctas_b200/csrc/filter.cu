@@ -43,16 +43,23 @@ template <int DIR> __device__ __forceinline__ float2 mul_i(float2 a) {
 // Twiddles w^q, q = 1 .. R-1, of butterfly m of a stage from its table entry
 // (w, w^4) (fbp_host.cpp, fft_twiddles_into: one 16-byte entry per butterfly
 // index, consecutive for consecutive m); w^2, w^3 and w^5..w^7 are at most two
-// complex products deep, a few ulps.
-template <int R>
-__device__ __forceinline__ void twiddles(const float4 *__restrict__ tws, int m, float2 *w) {
+// complex products deep, a few ulps.  FULL: all powers from the table (of plans with a
+// radix of 3, fft_twiddles with radices), two to an entry and h entries of each pair,
+// each rounded once.
+template <int R, bool FULL>
+__device__ __forceinline__ void twiddles(const float4 *__restrict__ tws, int m, int h, float2 *w) {
   const float4 e = __ldg(&tws[m]);
   w[1] = make_float2(e.x, e.y);
-  if (R == 3 || R == 5) {  // the entry is (w, w^2)
-    w[2] = make_float2(e.z, e.w);
-    if (R == 5) {
-      w[3] = cmul(w[2], w[1]);
-      w[4] = cmul(w[2], w[2]);
+  if (FULL) {
+#pragma unroll
+    for (int q = 2; q < R; q += 2) {
+      const float4 f = q == 2 ? e : __ldg(&tws[(q / 2 - 1) * h + m]);
+      if (q > 2) w[q - 1] = make_float2(f.x, f.y);
+      w[q] = make_float2(f.z, f.w);
+    }
+    if (R % 2 == 0 && R > 2) {
+      const float4 f = __ldg(&tws[(R / 2 - 1) * h + m]);
+      w[R - 1] = make_float2(f.x, f.y);
     }
     return;
   }
@@ -118,32 +125,15 @@ template <int DIR> __device__ __forceinline__ void dft3(float2 *x) {
   x[1] = a + b;
   x[2] = a - b;
 }
-template <int DIR> __device__ __forceinline__ void dft5(float2 *x) {
-  // cos 72, 144 = (-1 +- sqrt 5) / 4: in this form a constant row gives exact zeros
-  const float r = 0.55901699437494742410f;  // sqrt 5 / 4
-  const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;  // sin 72, 144
-  const float2 t1 = x[1] + x[4], t2 = x[2] + x[3], d1 = x[1] - x[4], d2 = x[2] - x[3];
-  const float2 t = t1 + t2, a = make_float2(x[0].x - 0.25f * t.x, x[0].y - 0.25f * t.y);
-  const float2 e = make_float2(r * (t1.x - t2.x), r * (t1.y - t2.y));
-  const float2 a1 = a + e, a2 = a - e;
-  const float2 b1 = mul_i<DIR>(make_float2(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y));
-  const float2 b2 = mul_i<DIR>(make_float2(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y));
-  x[0] = x[0] + t;
-  x[1] = a1 + b1;
-  x[4] = a1 - b1;
-  x[2] = a2 + b2;
-  x[3] = a2 - b2;
-}
 template <int R, int DIR> __device__ __forceinline__ void dft(float2 *x) {
   if (R == 2) dft2<DIR>(x);
   if (R == 3) dft3<DIR>(x);
-  if (R == 5) dft5<DIR>(x);
   if (R == 4) dft4<DIR>(x);
   if (R == 8) dft8<DIR>(x);
 }
 
 // Forward (decimation in frequency) stage of radix R, stride h, block R*h.
-template <int R>
+template <int R, bool FULL>
 __device__ void dif_stage(float2 *s, int P, int h, const float4 *__restrict__ tws) {
   // h is a power of two: block index b / h by a shift
   const int L = R * h, nb = P / R, lgh = __ffs(h) - 1;
@@ -155,7 +145,7 @@ __device__ void dif_stage(float2 *s, int P, int h, const float4 *__restrict__ tw
     dft<R, -1>(x);
     if (h > 1) {
       float2 w[R];
-      twiddles<R>(tws, m, w);
+      twiddles<R, FULL>(tws, m, h, w);
 #pragma unroll
       for (int q = 1; q < R; q++) x[q] = cmul(x[q], w[q]);
     }
@@ -165,7 +155,7 @@ __device__ void dif_stage(float2 *s, int P, int h, const float4 *__restrict__ tw
 }
 
 // Exact inverse of dif_stage (times R).
-template <int R>
+template <int R, bool FULL>
 __device__ void dit_stage(float2 *s, int P, int h, const float4 *__restrict__ tws) {
   // h is a power of two: block index b / h by a shift
   const int L = R * h, nb = P / R, lgh = __ffs(h) - 1;
@@ -176,7 +166,7 @@ __device__ void dit_stage(float2 *s, int P, int h, const float4 *__restrict__ tw
     for (int q = 0; q < R; q++) x[q] = s[sidx(base + q * h)];
     if (h > 1) {
       float2 w[R];
-      twiddles<R>(tws, m, w);
+      twiddles<R, FULL>(tws, m, h, w);
 #pragma unroll
       for (int q = 1; q < R; q++) x[q] = cmulc(x[q], w[q]);
     }
@@ -224,7 +214,7 @@ __device__ void middle_stage(float2 *s, int P, const float *__restrict__ gperm) 
 // First forward stage (one block of length P, stride h = P / R) with its
 // inputs produced by `ld(position)` -- read straight from global memory, so
 // each thread has R independent loads in flight.
-template <int R, class Loader>
+template <int R, bool FULL, class Loader>
 __device__ __forceinline__ void dif_first_stage(float2 *s, int h, const float4 *__restrict__ tws,
                                                 Loader ld) {
   for (int b = threadIdx.x; b < h; b += blockDim.x) {
@@ -233,7 +223,7 @@ __device__ __forceinline__ void dif_first_stage(float2 *s, int h, const float4 *
     for (int t = 0; t < R; t++) x[t] = ld(b + t * h);
     dft<R, -1>(x);
     float2 w[R];
-    twiddles<R>(tws, b, w);
+    twiddles<R, FULL>(tws, b, h, w);
 #pragma unroll
     for (int q = 1; q < R; q++) x[q] = cmul(x[q], w[q]);
 #pragma unroll
@@ -242,7 +232,7 @@ __device__ __forceinline__ void dif_first_stage(float2 *s, int h, const float4 *
 }
 
 // Last inverse stage with its outputs handed to `wr(position, value)`.
-template <int R, class Writer>
+template <int R, bool FULL, class Writer>
 __device__ __forceinline__ void dit_last_stage(const float2 *s, int h, const float4 *__restrict__ tws,
                                                Writer wr) {
   for (int b = threadIdx.x; b < h; b += blockDim.x) {
@@ -250,7 +240,7 @@ __device__ __forceinline__ void dit_last_stage(const float2 *s, int h, const flo
 #pragma unroll
     for (int q = 0; q < R; q++) x[q] = s[sidx(b + q * h)];
     float2 w[R];
-    twiddles<R>(tws, b, w);
+    twiddles<R, FULL>(tws, b, h, w);
 #pragma unroll
     for (int q = 1; q < R; q++) x[q] = cmulc(x[q], w[q]);
     dft<R, +1>(x);
@@ -259,16 +249,16 @@ __device__ __forceinline__ void dit_last_stage(const float2 *s, int h, const flo
   }
 }
 
-template <bool FWD>
+template <bool FWD, bool FULL>
 __device__ __forceinline__ void run_stage(float2 *s, int P, int R, int h, const float4 *tw) {
   if (FWD) {
-    if (R == 8) dif_stage<8>(s, P, h, tw);
-    else if (R == 4) dif_stage<4>(s, P, h, tw);
-    else dif_stage<2>(s, P, h, tw);
+    if (R == 8) dif_stage<8, FULL>(s, P, h, tw);
+    else if (R == 4) dif_stage<4, FULL>(s, P, h, tw);
+    else dif_stage<2, FULL>(s, P, h, tw);
   } else {
-    if (R == 8) dit_stage<8>(s, P, h, tw);
-    else if (R == 4) dit_stage<4>(s, P, h, tw);
-    else dit_stage<2>(s, P, h, tw);
+    if (R == 8) dit_stage<8, FULL>(s, P, h, tw);
+    else if (R == 4) dit_stage<4, FULL>(s, P, h, tw);
+    else dit_stage<2, FULL>(s, P, h, tw);
   }
 }
 
@@ -304,9 +294,9 @@ __device__ __forceinline__ float pow2_scale(float mx) {
 }
 
 // Filters rows 2*pair and 2*pair+1 of slice sl.  Called by every thread of
-// the CTA with the CTA's dynamic shared memory (P + P/16 float2).  ODD: P is 3 or 5
-// times a power of two, its first radix 3 or 5 (every later stride is a power of two).
-template <typename T, bool ODD = false>
+// the CTA with the CTA's dynamic shared memory (P + P/16 float2).  THREE: P is 3 times a
+// power of two, its first radix 3 (every later stride is a power of two).
+template <typename T, bool THREE = false>
 __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int sl) {
   extern __shared__ float2 sm[];
   __shared__ float red[2][kFftThreads / 32];
@@ -328,16 +318,21 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
     if (r1 + 1 < N) qb = deabs(qb, mm);
   }
 
-  // Periodic rows of odd plans are transformed less their mean, and the response to that
-  // constant is added back.  They fill the transform (two periods in 2n elements or
-  // little more), whose rounding is relative to what it holds: without this its error is
-  // 15 to 28 % above that of the next power of two.
+  // Periodic rows of these plans are transformed less their mean, and the response to
+  // that constant is added back; and every twiddle comes from the table, rounded once.
+  // The rounding error of a transform is relative to what its elements hold, and two
+  // periods fill 3 2^k of them to a larger part than the next power of two: without the
+  // first its error on rows with a mean, without the second on rows without one, is up
+  // to 15 % above that one's; with both it is 6 to 78 % below it (rows with and without a
+  // mean, derivatives, steps, noise and combs).  The mean is that of all samples, 9 % of
+  // the kernel's time: one of evenly spaced samples is wrong for a row of their period.
   float2 mean = make_float2(0.f, 0.f);
-  if (ODD && a.periodic) {
-    // one sample a thread, evenly spaced, is mean enough (all of them cost 17 % more)
-    const int c = threadIdx.x * W / (int)blockDim.x;
-    mean.x = abs_mode ? deabs(x0[c], mm) : x0[c];
-    if (has1) mean.y = abs_mode ? deabs(x1[c], mm) : x1[c];
+  if (THREE && a.periodic) {
+#pragma unroll 4
+    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+      mean.x += abs_mode ? deabs(x0[c], mm) : x0[c];
+      if (has1) mean.y += abs_mode ? deabs(x1[c], mm) : x1[c];
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       mean.x += __shfl_xor_sync(0xffffffffu, mean.x, o);
@@ -350,10 +345,10 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
     __syncthreads();
     mean = make_float2(0.f, 0.f);
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) mean = mean + make_float2(red[0][w], red[1][w]);
-    mean = make_float2(mean.x / (float)blockDim.x, mean.y / (float)blockDim.x);
+    mean = make_float2(mean.x / (float)W, mean.y / (float)W);
   }
   auto with_mean = [&](float2 z) {
-    return ODD && a.periodic ? make_float2(z.x + mean.x * a.dc, z.y + mean.y * a.dc) : z;
+    return THREE && a.periodic ? make_float2(z.x + mean.x * a.dc, z.y + mean.y * a.dc) : z;
   };
 
   // element p of the zero-padded row pair
@@ -372,7 +367,7 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
         v.x = deabs(v.x, mm);
         if (has1) v.y = deabs(v.y, mm);
       }
-      if (ODD && a.periodic) v = v - mean;
+      if (THREE && a.periodic) v = v - mean;
     } else if (c == W && !a.periodic) {
       v = make_float2(qa, qb);
     }
@@ -381,7 +376,8 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
 
   const int ns = a.nradix;
   int hs[8];
-  // twiddle table of stage st: tws + to[st] (h entries; fbp_host.cpp)
+  // twiddle table of stage st: tws + to[st] (h entries, with THREE h for every two
+  // powers; fbp_host.cpp)
   int to[8];
   const float4 *tws = reinterpret_cast<const float4 *>(a.tw);
   {
@@ -390,7 +386,7 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
       h /= a.radix[st];
       hs[st] = h;
       to[st] = o;
-      o += h;
+      o += THREE ? h * (a.radix[st] / 2) : h;
     }
   }
   // rows go straight from the last inverse stage to global memory unless a
@@ -407,17 +403,16 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
 
   if (ns >= 2) {
     const int R = a.radix[0];
-    if (ODD && R == 5) dif_first_stage<5>(sm, hs[0], tws, load);
-    else if (ODD) dif_first_stage<3>(sm, hs[0], tws, load);
-    else if (R == 8) dif_first_stage<8>(sm, hs[0], tws, load);
-    else if (R == 4) dif_first_stage<4>(sm, hs[0], tws, load);
-    else dif_first_stage<2>(sm, hs[0], tws, load);
+    if (THREE) dif_first_stage<3, true>(sm, hs[0], tws, load);
+    else if (R == 8) dif_first_stage<8, false>(sm, hs[0], tws, load);
+    else if (R == 4) dif_first_stage<4, false>(sm, hs[0], tws, load);
+    else dif_first_stage<2, false>(sm, hs[0], tws, load);
   } else {
     for (int p = threadIdx.x; p < P; p += blockDim.x) sm[sidx(p)] = load(p);
   }
   __syncthreads();
   for (int st = (ns >= 2 ? 1 : 0); st < ns - 1; st++) {
-    run_stage<true>(sm, P, a.radix[st], hs[st], tws + to[st]);
+    run_stage<true, THREE>(sm, P, a.radix[st], hs[st], tws + to[st]);
     __syncthreads();
   }
   {
@@ -428,12 +423,10 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
   }
   __syncthreads();
   for (int st = ns - 2; st >= (direct ? 1 : 0); st--) {
-    if (ODD && st == 0) {  // in place: every thread writes the elements that it read
-      auto keep = [&](int p, float2 v) { sm[sidx(p)] = with_mean(v); };
-      if (a.radix[0] == 5) dit_last_stage<5>(sm, hs[0], tws, keep);
-      else dit_last_stage<3>(sm, hs[0], tws, keep);
+    if (THREE && st == 0) {  // in place: every thread writes the elements that it read
+      dit_last_stage<3, true>(sm, hs[0], tws, [&](int p, float2 v) { sm[sidx(p)] = with_mean(v); });
     } else {
-      run_stage<false>(sm, P, a.radix[st], hs[st], tws + to[st]);
+      run_stage<false, THREE>(sm, P, a.radix[st], hs[st], tws + to[st]);
     }
     __syncthreads();
   }
@@ -463,11 +456,10 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
       }
     };
     const int R = a.radix[0];
-    if (ODD && R == 5) dit_last_stage<5>(sm, hs[0], tws, store);
-    else if (ODD) dit_last_stage<3>(sm, hs[0], tws, store);
-    else if (R == 8) dit_last_stage<8>(sm, hs[0], tws, store);
-    else if (R == 4) dit_last_stage<4>(sm, hs[0], tws, store);
-    else dit_last_stage<2>(sm, hs[0], tws, store);
+    if (THREE) dit_last_stage<3, true>(sm, hs[0], tws, store);
+    else if (R == 8) dit_last_stage<8, false>(sm, hs[0], tws, store);
+    else if (R == 4) dit_last_stage<4, false>(sm, hs[0], tws, store);
+    else dit_last_stage<2, false>(sm, hs[0], tws, store);
     return;
   }
 
@@ -571,7 +563,7 @@ __global__ void __launch_bounds__(kFftThreads) filter_rows_kernel(FilterLaunch a
   filter_pair<T>(a, blockIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(kFftThreads) filter_odd_kernel(FilterLaunch a) {
+__global__ void __launch_bounds__(kFftThreads) filter_three_kernel(FilterLaunch a) {
   filter_pair<float, true>(a, blockIdx.x, blockIdx.y);
 }
 
@@ -793,13 +785,13 @@ cudaError_t launch_filter_t(const FilterLaunch &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_filter_odd(const FilterLaunch &a, cudaStream_t st) {
+cudaError_t launch_filter_three(const FilterLaunch &a, cudaStream_t st) {
   if (a.store != 0 || a.quad || a.nradix < 2) return cudaErrorInvalidValue;
   const size_t smem = sizeof(float2) * (size_t)(a.P + a.P / 16);
   const cudaError_t e = cudaFuncSetAttribute(
-      filter_odd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      filter_three_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  filter_odd_kernel<<<dim3((a.N + 1) / 2, a.S), kFftThreads, smem, st>>>(a);
+  filter_three_kernel<<<dim3((a.N + 1) / 2, a.S), kFftThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -854,8 +846,8 @@ cudaError_t launch_expand_quad(const void *q, int64_t q_slice_stride, const floa
 }
 
 cudaError_t launch_filter(const FilterLaunch &a, cudaStream_t st) {
-  if (a.contrast != 3 && a.nradix > 0 && (a.radix[0] == 3 || a.radix[0] == 5))
-    return launch_filter_odd(a, st);
+  if (a.contrast != 3 && a.nradix > 0 && a.radix[0] == 3)
+    return launch_filter_three(a, st);
   if (a.quad && a.store != 0) return cudaErrorInvalidValue;
   if (a.quad && a.contrast != 3) return launch_filter_quad(a, st);
   if (a.store == 1) return launch_filter_t<__half>(a, st);

@@ -9,9 +9,12 @@
 // "periodic" mode) and multiplied by G_P = DFT_P(h), h the kernel g laid symmetrically
 // about 0 (|d| <= n/2; for even n the d = n/2 tap is split between +-n/2).  For outputs
 // n/2 .. 3n/2 - 1 every tap reads inside the two periods, so the result is the circular
-// convolution up to float rounding.  P is the least of 2^k, 3 2^k and 5 2^k: the filter
-// is bound by its passes over P elements in shared memory (5120 instead of 8192 for
-// rows of 2560).
+// convolution up to float rounding.  P is the lesser of 2^k and 3 2^k: the filter is
+// bound by its passes over P elements in shared memory (6144 instead of 8192 for rows
+// of 2560).  5 2^k (5120 there) ran in 0.94 ms where 3 2^k takes 1.16 ms on
+// 31 x 1024 x 2560, but its rounding error on rows whose mean is small against their
+// range is up to 10 % above that of 2^k, in every form of the twiddles and the mean
+// (filter.cu), and is not used.
 //
 // Backprojection.  One thread per result pixel adds the n images' terms in
 // order, with the reference's float expression for the sample index.
@@ -186,11 +189,9 @@ void ts_create(ctas_ts *h, int64_t rows, int64_t pixels, int32_t ftype, float fp
   h->P = ctas::padded_width(pixels);
   if (h->P > 16384)  // the row-pair FFT lives in shared memory
     ctas::fail(CTAS_E_UNSUPPORTED, "tomosynthesis: rows wider than 8192 pixels are not supported");
-  for (const int64_t odd : {3, 5}) {
-    int64_t P = 16 * odd;
-    while (P < 2 * pixels) P *= 2;
-    h->P = std::min(h->P, P);
-  }
+  int64_t three = 48;  // 3 2^k of at least two stages behind the radix of 3
+  while (three < 2 * pixels) three *= 2;
+  h->P = std::min(h->P, three);
   h->Wp = ctas::padded_pitch(pixels);
   // ts_add filters for every contrast; ABS adds -log, REF the running sum
   h->contrast = contrast == CTAS_FLT ? CTAS_PHS : contrast;
@@ -202,7 +203,7 @@ void ts_create(ctas_ts *h, int64_t rows, int64_t pixels, int32_t ftype, float fp
   std::vector<float> gp((size_t)h->P);
   for (int64_t p = 0; p < h->P; p++)
     gp[(size_t)p] = (float)(G[(size_t)perm[(size_t)p]] / (double)h->P);
-  const auto tw = ctas::fft_twiddles(h->P, h->radices);
+  const auto tw = h->radices[0] == 3 ? ctas::fft_twiddles(h->P, h->radices) : ctas::fft_twiddles(h->P);
   DevGuard g(dev);
   cuda_check(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
   h->tw.ensure(sizeof(float) * tw.size());
