@@ -725,7 +725,11 @@ constexpr int kRowPx = 130;                    // 128 output pixels + 2 halo
 constexpr int kRowChunkBytes = 17 * 1024;      // 130 x 128 B, padded to the 1 KB atom
 constexpr int kRowMaxSlots = 8;
 constexpr int kMaxAcc = 8;
-constexpr int kRowOut = 4 * 2 * kOutBytes;     // two staging buffers per epilogue warp
+// staging buffers per epilogue warp: one for 128 input channels, whose 128 -> 32 layer
+// fits shared memory only so (weights, four input rows and 8 KB of staging: 224,536 of
+// 232,448 bytes)
+__host__ __device__ constexpr int row_bufs(int cin) { return cin == 128 ? 1 : 2; }
+__host__ __device__ constexpr int row_out(int cin) { return 4 * row_bufs(cin) * kOutBytes; }
 
 struct RowArgs {
   const bf16 *mask;
@@ -776,7 +780,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t *slots = base;                                   // input-row ring (1 KB atoms)
   uint8_t *wsm = base + a.nslots * a.slot_bytes;           // weights
   uint8_t *outs = wsm + a.wbytes;                          // output staging
-  float *s_bias = reinterpret_cast<float *>(outs + kRowOut);
+  float *s_bias = reinterpret_cast<float *>(outs + row_out(CIN));
   uint64_t *row_full = reinterpret_cast<uint64_t *>(s_bias + kMaxCout);
   uint64_t *row_empty = row_full + kRowMaxSlots;
   uint64_t *acc_full = row_empty + kRowMaxSlots;  // [kMaxAcc]
@@ -987,8 +991,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * cout);
 #pragma unroll 1
         for (int c0 = 0; c0 < cout; c0 += 32, turn ^= 1) {
-          uint8_t *so = outs + (2 * q + turn) * kOutBytes;
-          drain32<1>(taddr + (uint32_t)c0, s_bias + c0, mp ? mp + c0 : nullptr, a.relu, so, lane);
+          constexpr int kBufs = row_bufs(CIN);
+          uint8_t *so = outs + (kBufs == 2 ? 2 * q + turn : q) * kOutBytes;
+          drain32<kBufs - 1>(taddr + (uint32_t)c0, s_bias + c0, mp ? mp + c0 : nullptr, a.relu, so, lane);
           if (lane == 0) tma_store_4d(&ymap, so, c0, sx * 128 + q * 32, y, b);
         }
         tc_fence_before();
@@ -1011,7 +1016,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                  : "memory");
 }
 
-constexpr int kRowSmemFixed = kRowOut + 4 * kMaxCout + (2 * kRowMaxSlots + 2 * kMaxAcc + 1) * 8 + 16 + 1024;  // bias, barriers, slack
+// bias, barriers, slack
+constexpr int kRowSmemFixed = 4 * kMaxCout + (2 * kRowMaxSlots + 2 * kMaxAcc + 1) * 8 + 16 + 1024;
 constexpr int kRowSmemMax = 232448, kRowSmemHalf = 233472 / 2 - 1024;
 
 // resident weights of the row form: 9 taps x cout rows x cin channels
@@ -1019,7 +1025,8 @@ int row_wbytes(const ConvArgs &a) { return 9 * a.cin * a.cout * 2; }
 
 // shared memory of the row form for `slots` input-row buffers
 int row_smem(const ConvArgs &a, int slots) {
-  return row_wbytes(a) + slots * ((a.cin + 63) / 64) * kRowChunkBytes + kRowSmemFixed;
+  return row_wbytes(a) + slots * ((a.cin + 63) / 64) * kRowChunkBytes + row_out(a.cin) +
+         kRowSmemFixed;
 }
 
 bool make_row_map(const ConvArgs &a, CUtensorMap *map) {
