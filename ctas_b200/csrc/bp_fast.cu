@@ -970,7 +970,9 @@ int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested, bool 
   if (env_tile() >= 0 && env_tile() < kTiles) return env_tile();
   int dev = 0;
   cudaGetDevice(&dev);
-  const TuneKey key = bp_fast_tune_key(a, dev, rest);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const TuneKey key = bp_fast_tune_key(a, dev, rest, sms);
   {
     std::lock_guard<std::mutex> g(g_tune_mutex);
     auto it = g_tuned.find(key);
@@ -979,6 +981,13 @@ int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested, bool 
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
+    std::lock_guard<std::mutex> g(g_tune_mutex);
+    for (const auto &e : g_tuned) {
+      TuneKey k = e.first;
+      std::get<8>(k) = rest;
+      std::get<9>(k) = std::get<9>(key);
+      if (k == key) return e.second;
+    }
     return kShapes * (kVariants - 1) + 1;
   }
   // time the candidates on a few slices of this launch (their output is
@@ -987,8 +996,6 @@ int bp_fast_choose_tile(const BpLaunch &a, cudaStream_t st, int requested, bool 
   // weighs on every candidate as it will on the real launch
   BpLaunch one = a;
   {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t tiles = (int64_t)((a.out_rows + 63) / 64) * ((a.out_cols + 127) / 128);
     const int64_t want = (8ll * 3 * sms + tiles - 1) / std::max<int64_t>(tiles, 1);
     one.S = (int)std::max<int64_t>(1, std::min<int64_t>(a.S, want));

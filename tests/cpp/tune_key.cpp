@@ -25,5 +25,13 @@ int main() {
     if (ctas::bp_fast_tune_key(b[i], 0, false) == key) return 10 + i;
   if (ctas::bp_fast_tune_key(a, 1, false) == key) return 20;
   if (ctas::bp_fast_tune_key(a, 0, true) == key) return 21;
+  // fill: slices of 700 x 700 (121 tiles of 64 x 64) on 148 SMs
+  ctas::BpLaunch c = a;
+  c.W = c.out_rows = c.out_cols = 700;
+  auto at = [&](int slices) {
+    c.S = slices;
+    return ctas::bp_fast_tune_key(c, 0, false, 148);
+  };
+  if (at(3) == at(5) || at(8) == at(9) || !(at(10) == at(40))) return 30;
   return 0;
 }
