@@ -37,6 +37,7 @@
 
 #include "bp_common.cuh"
 #include "bp_quad.hpp"
+#include "bp_quad_rule.hpp"
 #include "bp_stage.cuh"
 
 namespace ctas {
@@ -627,11 +628,6 @@ template <class TL> cudaError_t launch_form(const BpLaunch &a, cudaStream_t st, 
 
 const char *bp_quad_error_detail() { return t_detail; }
 
-bool bp_quad_pays(int64_t rows, int64_t cols, int64_t slices, int sms) {
-  const int64_t tiles = ((rows + QSmall::TY - 1) / QSmall::TY) * ((cols + QSmall::TX - 1) / QSmall::TX);
-  return 8 * tiles * ((slices + 3) / 4) >= 7 * (int64_t)sms;
-}
-
 cudaError_t launch_bp_quad(const BpLaunch &a, cudaStream_t st, bool check) {
   t_detail[0] = 0;
   int dev = 0, sms = 148;
@@ -640,7 +636,8 @@ cudaError_t launch_bp_quad(const BpLaunch &a, cudaStream_t st, bool check) {
   if (a.interp == 1 && a.wide) return cudaErrorInvalidValue;
   const int64_t tiles = (int64_t)((a.out_rows + QLarge::TY - 1) / QLarge::TY) *
                         ((a.out_cols + QLarge::TX - 1) / QLarge::TX) * ((a.S + 3) / 4);
-  return 2 * tiles < 3 * sms ? launch_form<QSmall>(a, st, check) : launch_form<QLarge>(a, st, check);
+  return quad_small_tile(tiles, sms) ? launch_form<QSmall>(a, st, check)
+                                     : launch_form<QLarge>(a, st, check);
 }
 
 }  // namespace ctas

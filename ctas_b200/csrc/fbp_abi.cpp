@@ -31,6 +31,7 @@
 #include "../../include/ctas_volume.h"
 #include "bp_fast.hpp"
 #include "bp_quad.hpp"
+#include "bp_quad_rule.hpp"
 #include "fbp_host.hpp"
 #include "fbp_kernels.hpp"
 
@@ -119,6 +120,11 @@ struct Consts {
   }
 };
 
+// Slices of the one-slice kernel and groups that a launch may need (quad_need).
+struct QuadNeed {
+  int64_t alone, groups;
+};
+
 // One set of work buffers (the host stack call double-buffers two sets).
 struct WorkSet {
   DevBuf raw, filt, scale, slice, part, minmax, ring_avg, ring;
@@ -156,6 +162,8 @@ struct ctas_fbp {
   bool wide = false;
   int64_t off = ctas::kRowOff;
   int device = 0, sms = 148;
+  ctas::SliceTiles tiles;
+  std::vector<QuadNeed> need;  // quad_need(), by slice count, as far as asked for
   std::shared_ptr<Consts> dc;
   cudaStream_t stream = nullptr, s_in = nullptr, s_out = nullptr;
   WorkSet ws[2];
@@ -253,25 +261,43 @@ void init_streams(ctas_fbp *h) {
 // bounded number at a time.
 bool quad_capable(const ctas_fbp *h) {
   return (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
-         !ctas::bp_fast_tile_forced();
+         h->tiles.in64 > 0 && !ctas::bp_fast_tile_forced();
 }
 
-// How many of S slices (the first ones) go through the four-slice kernel: whole
-// groups, and a group of the last three.  One or two slices left over take the
-// one-slice kernel (a group's time is that of 2.2 slices of 1800 x 2560 alone), unless
-// they are so small that a launch of their own leaves most of the device idle: the last
-// slice of 29 of 1784 x 296 takes 230 us alone and 115 us as a group more.
+ctas::QuadForm quad_form(const ctas_fbp *h) {
+  return h->interp == CTAS_INTERP_LINEAR ? ctas::kQuadLinear : h->wide ? ctas::kQuadWide : ctas::kQuadTrunc;
+}
+
+// How many of S slices (the first ones) go through the four-slice kernel: those that
+// quad_slices() (bp_quad_rule.hpp) estimates to run faster in groups.  The test aid
+// groups all of them but a rest of one or two, which joins where slices are small.
 int64_t quad_count(const ctas_fbp *h, int64_t S) {
   if (S < 3 || !quad_capable(h)) return 0;
-  const int64_t rest = S % ctas::kQuadSlices;
-  const bool small = ((h->out_rows + 63) / 64) * ((h->out_cols + 63) / 64) <= 48;
-  const int64_t n = rest == 3 || small ? S : S - rest;
-  if (!(h->flags & CTAS_FLAG_GROUPS) && !ctas::bp_quad_pays(h->out_rows, h->out_cols, n, h->sms))
-    return 0;
-  return n;
+  if (h->flags & CTAS_FLAG_GROUPS)
+    return S % ctas::kQuadSlices == 3 || h->tiles.all64 <= 48 ? S : S - S % ctas::kQuadSlices;
+  return ctas::quad_slices(quad_form(h), h->tiles, S, h->sms);
 }
 
 int64_t quad_groups(int64_t slices) { return (slices + ctas::kQuadSlices - 1) / ctas::kQuadSlices; }
+
+// Most slices that one launch of at most S slices leaves to the one-slice kernel, and
+// most groups that it forms.  Neither is that of S: five slices may be grouped where six
+// are not.  Buffers sized by these serve every smaller count, without an allocation that
+// a capture of one would refuse.
+QuadNeed quad_need(ctas_fbp *h, int64_t S) {
+  if (!quad_capable(h)) return {S, 0};
+  if (h->flags & CTAS_FLAG_GROUPS) return {std::min<int64_t>(S, 2), S < 3 ? 0 : quad_groups(S)};
+  const int64_t last = ctas::quad_always(h->tiles, h->sms);
+  std::vector<QuadNeed> &v = h->need;
+  for (int64_t s = (int64_t)v.size(); s <= std::min(S, last); s++) {
+    const int64_t n = quad_count(h, s);
+    QuadNeed q{s - n, quad_groups(n)};
+    if (s > 0) q = {std::max(q.alone, v.back().alone), std::max(q.groups, v.back().groups)};
+    v.push_back(q);
+  }
+  if (S <= last) return v[(size_t)S];
+  return {std::max<int64_t>(3, v[(size_t)last].alone), std::max(quad_groups(S), v[(size_t)last].groups)};
+}
 
 // Groups that the interleaved buffer holds: all of them for float32 rows, which the
 // filter stores there; for 16-bit rows as many as 512 MB take, expanded in turn.
@@ -292,14 +318,10 @@ float *quad_rows(const WorkSet &w) {
 void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw, cudaStream_t st) {
   const int64_t N = h->N, W = h->W;
   if (need_raw) w.raw.ensure(sizeof(float) * (size_t)(S * N * W));
-  const int64_t n4 = quad_count(h, S);
-  // most slices that a launch of at most S leaves to the one-slice kernel: those below
-  // the first count that forms groups, or a rest of two
-  int64_t alone = S;
-  if (n4 > 0 && h->store == CTAS_STORE_F32)
-    for (alone = 2; quad_count(h, alone + 1) == 0;) alone++;
-  if (n4 > 0) {
-    const int64_t words = quad_resident(h, quad_groups(S)) * N * h->Wp + 2 * ctas::kQuadSlack;
+  const QuadNeed need = quad_need(h, S);
+  const int64_t alone = h->store == CTAS_STORE_F32 ? need.alone : S;
+  if (need.groups > 0) {
+    const int64_t words = quad_resident(h, need.groups) * N * h->Wp + 2 * ctas::kQuadSlack;
     if (w.quad.ensure(sizeof(float) * ctas::kQuadSlices * (size_t)words))
       cuda_check(cudaMemsetAsync(w.quad.p, 0, w.quad.bytes, st), "cudaMemsetAsync");
   }
@@ -867,6 +889,7 @@ int ctas_fbp_create(ctas_fbp **out, int64_t n_angles, int64_t width, int32_t con
     DeviceGuard g(h->device);
     cuda_check(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device),
                "cudaDeviceGetAttribute");
+    h->tiles = ctas::slice_tiles(width, h->out_rows, h->out_cols, h->geo_oj, h->geo_oi, h->geo_p);
 
     // constants: twiddles, window in the FFT's output order (divided by P),
     // angle table
@@ -945,6 +968,7 @@ int ctas_fbp_clone(const ctas_fbp *src, ctas_fbp **out) {
     h->off = src->off;
     h->device = src->device;
     h->sms = src->sms;
+    h->tiles = src->tiles;
     h->dc = src->dc;
     init_streams(h.get());
     *out = h.release();
