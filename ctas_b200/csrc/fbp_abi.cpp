@@ -632,17 +632,6 @@ int64_t device_chunk(const ctas_fbp *h, int64_t S) {
   return whole_groups(h, S, (S + nch - 1) / nch);
 }
 
-int64_t host_chunk(const ctas_fbp *h, int64_t S) {
-  if (h->chunk > 0) return std::min<int64_t>(h->chunk, S);
-  const double per = (double)h->N * h->W * 4 + (double)h->N * h->Wp * elem_bytes(h->store) +
-                     4.0 * h->out_rows * h->out_cols;
-  int64_t cmax = std::max<int64_t>(1, (int64_t)(1.0e9 / per));
-  // keep at least a few chunks so copies overlap compute
-  cmax = std::min<int64_t>(cmax, std::max<int64_t>(1, (S + 3) / 4));
-  const int64_t nch = (S + cmax - 1) / cmax;
-  return whole_groups(h, S, (S + nch - 1) / nch);
-}
-
 // Chunk sizes of the host stack call: chunks of C slices, entered and left
 // through chunks of 2, 4, 8, ... slices, so that the first upload and the last
 // download (the copies no compute overlaps) are short.  unit: chunks but the last of the
@@ -663,6 +652,55 @@ std::vector<int64_t> chunk_plan(int64_t n, int64_t C, int64_t unit) {
     if (edge(i + 1) > edge(i)) plan.push_back(edge(i + 1) - edge(i));
   plan.insert(plan.end(), up.rbegin(), up.rend());
   return plan;
+}
+
+// Estimated time of the host stack call's pipeline over `plan`, us: upload, compute and
+// download run beside one another, and a chunk's upload waits for the download two
+// chunks before it, whose buffers it takes.  Copies at 50 GB/s each way from and to
+// pinned memory and 12 GB/s else, where they return only when they are done; filters at
+// their measured rate (90 us per 1800 x 2560 slice at 8192 points).
+double plan_us(const ctas_fbp *h, const std::vector<int64_t> &plan, bool wb, bool pinned) {
+  const double bytes_us = pinned ? 50e3 : 12e3;
+  const double NW = (double)h->N * h->W, OO = (double)h->out_rows * h->out_cols;
+  const double filter = h->contrast == CTAS_FLT ? 0.0 : 4.7e-7 * h->N * h->P * std::log2((double)h->P);
+  double in = 0, done = 0, out = 0, out_before = 0;
+  for (const int64_t S : plan) {
+    in = std::max(in, pinned ? out_before : out) + 4.0 * S * NW / bytes_us;
+    done = std::max(done, in) + 10.0 + S * filter +
+           h->N / 720.0 * ctas::stack_us(quad_form(h), h->tiles, S, quad_count(h, S), h->sms, 1.08);
+    out_before = out;
+    out = std::max(out, done) + 4.0 * S * (OO + (wb ? NW : 0.0)) / bytes_us;
+  }
+  return out;
+}
+
+// Chunks of the host calls.  Groups of four need chunks of at least four slices, whose
+// copies overlap less: four slices of 180 x 4096, bound by their copies, took 6.7 ms in
+// one chunk and 5.5 ms in four.  The faster of both is taken, by estimate.
+struct HostPlan {
+  int64_t C, unit;  // slices per chunk; chunks are multiples of unit
+};
+HostPlan host_plan(const ctas_fbp *h, int64_t S, bool wb, bool pinned) {
+  if (h->chunk > 0) return {std::min<int64_t>(h->chunk, S), 1};
+  const double per = (double)h->N * h->W * 4 + (double)h->N * h->Wp * elem_bytes(h->store) +
+                     4.0 * h->out_rows * h->out_cols;
+  int64_t cmax = std::max<int64_t>(1, (int64_t)(1.0e9 / per));
+  // keep at least a few chunks so copies overlap compute
+  cmax = std::min<int64_t>(cmax, std::max<int64_t>(1, (S + 3) / 4));
+  const int64_t nch = (S + cmax - 1) / cmax, C = (S + nch - 1) / nch, u = ctas::kQuadSlices;
+  const int64_t G = std::min(S, quad_groups(C) * u);
+  if (quad_count(h, G) == 0) return {C, 1};
+  if ((h->flags & CTAS_FLAG_GROUPS) ||
+      plan_us(h, chunk_plan(S, G, u), wb, pinned) < 0.97 * plan_us(h, chunk_plan(S, C, 1), wb, pinned))
+    return {G, u};
+  return {C, 1};
+}
+
+bool is_pinned(const void *p) {
+  cudaPointerAttributes at{};
+  const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess;
+  cudaGetLastError();
+  return ok && at.type != cudaMemoryTypeUnregistered;
 }
 
 // A closable blocking queue between the volume call's threads.
@@ -1197,12 +1235,15 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     if (!sinos || !slices) ctas::fail(CTAS_E_ARG, "null buffer");
     check_center(h, center);
     DeviceGuard g(h->device);
-    const int64_t C = host_chunk(h, n_slices);
     const bool wb = !(h->flags & CTAS_FLAG_NO_WRITEBACK);
+    const HostPlan hp = host_plan(h, n_slices, wb, is_pinned(sinos) && is_pinned(slices));
+    const int64_t C = hp.C;
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
     // four-slice groups are filtered into interleaved rows: the rows to write back are
     // stored densely beside them
-    const bool dense = wb && h->store == CTAS_STORE_F32 && quad_count(h, C) > 0;
+    const std::vector<int64_t> plan = chunk_plan(n_slices, C, hp.unit);
+    const bool dense = wb && h->store == CTAS_STORE_F32 &&
+                       std::any_of(plan.begin(), plan.end(), [&](int64_t S) { return quad_count(h, S) > 0; });
     for (auto &w : h->ws) {
       ensure_set(h, w, C, true, h->stream);
       if (dense) w.dense.ensure(sizeof(float) * (size_t)(C * NW));
@@ -1234,8 +1275,6 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     }
     // three-stream pipeline: host->device (s_in), compute (stream),
     // device->host (s_out); two work sets alternate.
-    const bool groups = h->chunk <= 0 && quad_count(h, n_slices) > 0;
-    const std::vector<int64_t> plan = chunk_plan(n_slices, C, groups ? ctas::kQuadSlices : 1);
     int64_t k = 0, s0 = 0;
     for (const int64_t S : plan) {
       WorkSet &w = h->ws[k & 1];
@@ -1303,7 +1342,7 @@ int ctas_fbp_reconstruct_volume(ctas_fbp *h, int64_t n_slices, float center, int
     if (n_slices == 0) return CTAS_OK;
     check_center(h, center);
     DeviceGuard g(h->device);
-    const int64_t C = host_chunk(h, n_slices);
+    const int64_t C = host_plan(h, n_slices, false, true).C;  // through the pinned rings
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
     const bool own_range = bpp != 0 && mincon == maxcon;
     for (auto &w : h->ws) {
