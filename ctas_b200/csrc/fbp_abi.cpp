@@ -164,6 +164,7 @@ struct ctas_fbp {
   int device = 0, sms = 148;
   ctas::SliceTiles tiles;
   std::vector<QuadNeed> need;  // quad_need(), by slice count, as far as asked for
+  bool singles = false;        // while a call runs without groups for want of memory
   std::shared_ptr<Consts> dc;
   cudaStream_t stream = nullptr, s_in = nullptr, s_out = nullptr;
   WorkSet ws[2];
@@ -261,7 +262,7 @@ void init_streams(ctas_fbp *h) {
 // bounded number at a time.
 bool quad_capable(const ctas_fbp *h) {
   return (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
-         h->tiles.in64 > 0 && !ctas::bp_fast_tile_forced();
+         h->tiles.in64 > 0 && !h->singles && !ctas::bp_fast_tile_forced();
 }
 
 ctas::QuadForm quad_form(const ctas_fbp *h) {
@@ -339,6 +340,33 @@ void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw, cudaStream_t 
   }
   w.slices = std::max(w.slices, S);
 }
+
+// Buffers of a stack call: size() chooses the chunks and allocates for them.  Where the
+// buffers of groups do not fit the device, the call runs one slice at a time, as long as
+// this object lives.
+struct StackBuffers {
+  ctas_fbp *h;
+  template <class F> StackBuffers(ctas_fbp *handle, F &&size) : h(handle) {
+    try {
+      size();
+    } catch (const ctas::Error &e) {
+      if (e.code != CTAS_E_NOMEM || !quad_capable(h)) throw;
+      for (auto &w : h->ws) {
+        w.quad.release();
+        w.dense.release();
+      }
+      h->singles = true;
+      try {
+        size();
+      } catch (...) {
+        h->singles = false;
+        throw;
+      }
+    }
+  }
+  ~StackBuffers() { h->singles = false; }
+  StackBuffers(const StackBuffers &) = delete;
+};
 
 void check_center(const ctas_fbp *h, float center) {
   // abs(center) >= ish(1)/2 (lct.cpp:614, 651): integer half width
@@ -682,7 +710,10 @@ struct HostPlan {
 };
 HostPlan host_plan(const ctas_fbp *h, int64_t S, bool wb, bool pinned) {
   if (h->chunk > 0) return {std::min<int64_t>(h->chunk, S), 1};
-  const double per = (double)h->N * h->W * 4 + (double)h->N * h->Wp * elem_bytes(h->store) +
+  // a chunk's buffers in at most 1 GB: rows, filtered rows (and their dense copy where
+  // groups are written back), slices
+  const bool dense = wb && h->store == CTAS_STORE_F32 && quad_capable(h);
+  const double per = (double)h->N * h->W * (dense ? 8 : 4) + (double)h->N * h->Wp * elem_bytes(h->store) +
                      4.0 * h->out_rows * h->out_cols;
   int64_t cmax = std::max<int64_t>(1, (int64_t)(1.0e9 / per));
   // keep at least a few chunks so copies overlap compute
@@ -1213,9 +1244,12 @@ int ctas_fbp_reconstruct_stack_dev(ctas_fbp *h, const float *sinos_dev, float *s
     check_center(h, center);
     DeviceGuard g(h->device);
     cudaStream_t st = (cudaStream_t)stream;
-    const int64_t C = device_chunk(h, n_slices);
     WorkSet &w = h->ws[0];
-    ensure_set(h, w, C, false, st);
+    int64_t C = 0;
+    StackBuffers sized(h, [&] {
+      C = device_chunk(h, n_slices);
+      ensure_set(h, w, C, false, st);
+    });
     for (int64_t s0 = 0; s0 < n_slices; s0 += C) {
       const int64_t S = std::min(C, n_slices - s0);
       run_filter(h, sinos_dev + s0 * h->N * h->W, S, w, st);
@@ -1236,18 +1270,24 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
     check_center(h, center);
     DeviceGuard g(h->device);
     const bool wb = !(h->flags & CTAS_FLAG_NO_WRITEBACK);
-    const HostPlan hp = host_plan(h, n_slices, wb, is_pinned(sinos) && is_pinned(slices));
-    const int64_t C = hp.C;
+    const bool pinned = is_pinned(sinos) && is_pinned(slices);
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
-    // four-slice groups are filtered into interleaved rows: the rows to write back are
-    // stored densely beside them
-    const std::vector<int64_t> plan = chunk_plan(n_slices, C, hp.unit);
-    const bool dense = wb && h->store == CTAS_STORE_F32 &&
-                       std::any_of(plan.begin(), plan.end(), [&](int64_t S) { return quad_count(h, S) > 0; });
-    for (auto &w : h->ws) {
-      ensure_set(h, w, C, true, h->stream);
-      if (dense) w.dense.ensure(sizeof(float) * (size_t)(C * NW));
-    }
+    int64_t C = 0;
+    std::vector<int64_t> plan;
+    bool dense = false;
+    StackBuffers sized(h, [&] {
+      const HostPlan hp = host_plan(h, n_slices, wb, pinned);
+      C = hp.C;
+      plan = chunk_plan(n_slices, C, hp.unit);
+      // four-slice groups are filtered into interleaved rows: the rows to write back are
+      // stored densely beside them
+      dense = wb && h->store == CTAS_STORE_F32 &&
+              std::any_of(plan.begin(), plan.end(), [&](int64_t S) { return quad_count(h, S) > 0; });
+      for (auto &w : h->ws) {
+        ensure_set(h, w, C, true, h->stream);
+        if (dense) w.dense.ensure(sizeof(float) * (size_t)(C * NW));
+      }
+    });
     // If a later chunk fails, copies of earlier chunks into the caller's host
     // buffers may still be queued: drain all three streams before returning,
     // so the caller may free those buffers once the call has returned.
@@ -1342,17 +1382,20 @@ int ctas_fbp_reconstruct_volume(ctas_fbp *h, int64_t n_slices, float center, int
     if (n_slices == 0) return CTAS_OK;
     check_center(h, center);
     DeviceGuard g(h->device);
-    const int64_t C = host_plan(h, n_slices, false, true).C;  // through the pinned rings
     const int64_t NW = h->N * h->W, OO = h->out_rows * h->out_cols;
     const bool own_range = bpp != 0 && mincon == maxcon;
-    for (auto &w : h->ws) {
-      ensure_set(h, w, C, true, h->stream);
-      if (bpp != 0) w.samples.ensure((size_t)(sb * C * OO));
-      if (own_range) {
-        w.part.ensure(sizeof(float2) * (size_t)(C * ctas::kMinMaxBlocks));
-        w.minmax.ensure(sizeof(float2) * (size_t)C);
+    int64_t C = 0;
+    StackBuffers sized(h, [&] {
+      C = host_plan(h, n_slices, false, true).C;  // through the pinned rings
+      for (auto &w : h->ws) {
+        ensure_set(h, w, C, true, h->stream);
+        if (bpp != 0) w.samples.ensure((size_t)(sb * C * OO));
+        if (own_range) {
+          w.part.ensure(sizeof(float2) * (size_t)(C * ctas::kMinMaxBlocks));
+          w.minmax.ensure(sizeof(float2) * (size_t)C);
+        }
       }
-    }
+    });
     for (int i = 0; i < 3; i++) {
       ensure_host(h->vin[i], sizeof(float) * (size_t)(C * NW));
       ensure_host(h->vout[i], (size_t)(sb * C * OO));

@@ -217,7 +217,16 @@ int ctas_fbp_synchronize(ctas_fbp *h);
  * centre (the ct tool's slice loop, ct.cpp:170-206).  Host form: pipelined
  * host->device, compute and device->host copies; sinos_inout receives the
  * filtered sinograms unless CTAS_FLAG_NO_WRITEBACK.  Device form: contiguous
- * [n_slices][N][W] input and [n_slices][rows][cols] output. */
+ * [n_slices][N][W] input and [n_slices][rows][cols] output.
+ * Device memory, kept by the handle until it is destroyed.  Stacks may be
+ * reconstructed four slices at a time, from filtered rows held as float32
+ * whatever `store` is.  Device form: the filtered rows of a chunk, up to 4 GB
+ * in `store` (and at least four slices), its slices, and with a 16-bit store
+ * up to 512 MB of float32 rows.  Host form: two sets of a chunk's rows,
+ * filtered rows (twice with write-back, for whole groups) and slices, up to
+ * 1 GB each (and at least four slices), and with a 16-bit store up to 512 MB
+ * of float32 rows each.  Where this does not fit, the call runs one slice at a
+ * time in the buffers of that form. */
 int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos_inout, float *slices_out,
                                int64_t n_slices, float center);
 int ctas_fbp_reconstruct_stack_dev(ctas_fbp *h, const float *sinos_dev,
