@@ -1796,7 +1796,6 @@ int ctas_fbp_batch_create(ctas_fbp_batch **out, const ctas_fbp_job *jobs, int64_
     b->n_pairs = pairs;
     if (row * Wp > ((int64_t)1 << 34)) ctas::fail(CTAS_E_SHAPE, "batch too large");
     b->filt.ensure(sizeof(float) * (size_t)(row * Wp));
-    cuda_check(cudaMemset(b->filt.p, 0, b->filt.bytes), "cudaMemset");
     b->tables.ensure(sizeof(float) * host.size());
     cuda_check(cudaMemcpy(b->tables.p, host.data(), sizeof(float) * host.size(),
                           cudaMemcpyHostToDevice),
@@ -1821,9 +1820,11 @@ int ctas_fbp_batch_create(ctas_fbp_batch **out, const ctas_fbp_job *jobs, int64_
     b->d_bjobs.ensure(sizeof(ctas::BatchJob) * b->bjobs.size());
     b->counter.ensure(sizeof(int));
     b->err.ensure(sizeof(int));
-    cuda_check(cudaMemset(b->err.p, 0, sizeof(int)), "cudaMemset");
     cuda_check(cudaMallocHost((void **)&b->err_host, sizeof(int)), "cudaMallocHost");
     cuda_check(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    // a plain cudaMemset returns before it has run
+    zero_now(b->filt.p, b->filt.bytes, b->stream);
+    zero_now(b->err.p, sizeof(int), b->stream);
 
     // autotune the tile on this batch (timing the whole filter + backprojection)
     const int ntiles = ctas::bp_fast_tile_count();
@@ -1936,7 +1937,7 @@ int ctas_fbp_batch_synchronize(ctas_fbp_batch *b) {
     cuda_check(cudaMemcpy(b->err_host, b->err.p, sizeof(int), cudaMemcpyDeviceToHost), "cudaMemcpy");
     const int w = *b->err_host;
     if (w) {
-      cuda_check(cudaMemset(b->err.p, 0, sizeof(int)), "cudaMemset");
+      zero_now(b->err.p, sizeof(int), b->stream);
       if (w & 4) ctas::fail(CTAS_E_TIMEOUT, "a device wait timed out in the backprojection kernel");
       ctas::fail(CTAS_E_CUDA, "device error word " + std::to_string(w));
     }

@@ -440,8 +440,9 @@ void create(ctas_unet *u, uint64_t seed, int32_t device) {
   u->parb.ensure(sizeof(bf16) * (size_t)u->npar);
   u->flip.ensure(sizeof(bf16) * (size_t)u->npar);
   cuda_check(cudaMemcpy(u->par.p, p.data(), fb, cudaMemcpyHostToDevice), "cudaMemcpy");
-  cuda_check(cudaMemset(u->m.p, 0, fb), "cudaMemset");
-  cuda_check(cudaMemset(u->v.p, 0, fb), "cudaMemset");
+  // on the stream that is waited for below: a plain cudaMemset returns before it has run
+  cuda_check(cudaMemsetAsync(u->m.p, 0, fb, u->stream), "cudaMemsetAsync");
+  cuda_check(cudaMemsetAsync(u->v.p, 0, fb, u->stream), "cudaMemsetAsync");
   refresh_bf16(u, u->stream);
   cuda_check(cudaStreamSynchronize(u->stream), "cudaStreamSynchronize");
 }

@@ -62,3 +62,25 @@ def test_first_stack_beside_busy_legacy_stream(cycles, store):
             out.append(_bits(y))
             torch.cuda.synchronize()
     assert np.array_equal(out[0], out[1])
+
+
+def test_batch_made_beside_busy_legacy_stream():
+    """A batch made and run on a side stream while the legacy stream is busy."""
+    import torch
+    x = torch.from_numpy(_rows(3)).cuda()
+    out = []
+    for busy in (0, 40_000_000):
+        y = torch.full((2, W, W), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()
+        if busy:
+            torch.cuda._sleep(busy)
+        with torch.cuda.stream(side):
+            batch = ct.Batch([(x[0], y[0], C), (x[1], y[1], -C)], ct.Contrast.PHS, 180.0,
+                             ct.Filter("HANN"))
+            batch.run()
+        side.synchronize()
+        out.append(_bits(y))
+        batch.close()
+        torch.cuda.synchronize()
+    assert np.array_equal(out[0], out[1])
