@@ -194,24 +194,9 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-// D[tmem] (+)= A[desc] * B[desc]^T, kind::f16 (BF16 operands, FP32 accumulate)
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same by a whole converged warp, whose elected lane issues: descriptors and
-// loop counters stay warp-uniform, in uniform registers.
+// D[tmem] (+)= A[desc] * B[desc]^T, kind::f16 (BF16 operands, FP32 accumulate), by a
+// whole converged warp, whose elected lane issues: descriptors and loop counters stay
+// warp-uniform, in uniform registers.
 __device__ __forceinline__ void tc_mma_w(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
