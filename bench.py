@@ -221,13 +221,32 @@ def cpu_reference_sample(sino: np.ndarray, target_s: float, threads: int,
 
 
 # ------------------------------------------------------------------ roofline
+def quad_loads_per_update():
+    """Shared-memory loads per pixel and projection of the four-slice kernel over this
+    workload's angles: a thread's eight pixels take 3 to 8 loads, by how far t moves along
+    the slower (u) and the faster axis (s) (sharing patterns, csrc/bp_quad.cu)."""
+    import oracle as O
+    tab = np.abs(O.angle_table(180.0, N_ANGLES).reshape(-1, 2).astype(np.float64))
+    u, s, m = tab.min(1), tab.max(1), (WIDTH + 256) * 2.0 ** -19
+    along = (s <= 1 - m) & (u + m <= s)
+    loads = np.where(3 * u <= 1 - m, 4, 8)
+    loads = np.where(along & (s + m <= 2 * u), np.where(3 * u - s <= 1 - m, 4, 5), loads)
+    loads = np.where(along & (2 * u + m <= s) & (2 * u <= 1 - m) & (s + m <= 3 * u), 4, loads)
+    loads = np.where(along & (3 * u + m <= s) & (3 * u <= 1 - m), 3, loads)
+    return float(loads.mean()) / 8.0
+
+
 def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_peak_gbs,
              clocks, sms, l2_peak_gbs=None, tile=None):
     import oracle as O
     from ctas_b200 import ct
     mask = O.mask(WIDTH, CENTER)
     inmask = int(mask.sum())
-    bp_bytes = 4.0 * N_ANGLES * inmask * slices_per_launch    # 4 B fetched per update
+    groups = tile is not None and tile < 0   # no tile id: the four-slice kernel
+    # 4 B fetched per update; in groups 16 B serve the updates of four slices, and a load
+    # those of several pixels
+    loads = quad_loads_per_update() if groups else 1.0
+    bp_bytes = 4.0 * loads * N_ANGLES * inmask * slices_per_launch
     achieved = bp_bytes / (bp_ms_per_launch * 1e-3) / 1e9
     # detector windows the staged kernel copies from L2 by TMA: one window of
     # `box` samples per projection for every tile that has a pixel in the disc
@@ -242,7 +261,6 @@ def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_pea
               "peak": round(l2_peak_gbs, 1), "frac": round(l2_ach / l2_peak_gbs, 4),
               "unit": "GB/s", "peak_source": "measured in this run by ctas_probe_l2_read "
                                             "(16-byte L2 reads of a 32 MiB buffer)"}
-    groups = tile is not None and tile < 0   # no tile id: the four-slice kernel
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if os.path.exists(tpath):
@@ -290,9 +308,10 @@ def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_pea
                           "this kernel (profiles/ncu_traffic.json, per slice, scaled to the "
                           "launch): a committed measurement, not taken in this run",
         "algorithmic_bytes_per_launch": bp_bytes,
-        "unit_note": "4 B per in-mask update (N x in-mask pixels per slice)" +
-                     ("; a sample may serve several pixels (0.49 loads per pixel), so this "
-                      "bound of one load per update can be exceeded" if groups else ""),
+        "loads_per_update": round(loads, 4),
+        "unit_note": "4 B x loads_per_update per in-mask update (N x in-mask pixels per "
+                     "slice)" + ("; loads shared between pixels, 16 B for four slices"
+                                 if groups else ""),
         "filter": {"bound": "hbm", "unit": "GB/s",
                    "achieved": round(f_ach, 1) if f_ach else None, "peak": hbm_peak,
                    "frac": round(f_ach / hbm_peak, 4) if f_ach else None,
@@ -505,19 +524,19 @@ def main():
 
     if rank == 0:
         # the graded fraction of the whole step: t_bound / t_measured per slice,
-        # t_bound = max(compulsory HBM bytes / HBM peak, dense updates x 4 B /
-        # nominal shared-memory fetch peak at the maximum SM clock)
+        # t_bound = max(compulsory HBM bytes / HBM peak, dense updates x 4 B x loads per
+        # update / nominal shared-memory fetch peak at the maximum SM clock)
         hbm_b = 4.0 * N_ANGLES * WIDTH * 3 + 4.0 * WIDTH * WIDTH + 8.0 * N_ANGLES
         fetch_peak = 128.0 * props.multi_processor_count * (clocks.get("sm_max_mhz") or 1965.0) * 1e6
         t_bound = max(hbm_b / (roof["filter"]["peak"] * 1e9),
-                      4.0 * N_ANGLES * WIDTH * WIDTH / fetch_peak)
+                      4.0 * roof["loads_per_update"] * N_ANGLES * WIDTH * WIDTH / fetch_peak)
         t_meas = (ms / args.steps) * 1e-3 / S
         roof["step_graded"] = {
             "t_bound_ms_per_slice": round(t_bound * 1e3, 4),
             "t_measured_ms_per_slice": round(t_meas * 1e3, 4),
             "frac": round(t_bound / t_meas, 4),
             "fetch_peak_gbs": round(fetch_peak / 1e9, 1),
-            "convention": "dense N x W^2 updates at 4 B each against 128 B/clk/SM at the "
+            "convention": "dense N x W^2 updates at 4 B x loads_per_update each against 128 B/clk/SM at the "
                           "maximum SM clock; HBM term: raw read, filtered write and read, "
                           "slice write"}
         line = {
