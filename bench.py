@@ -266,8 +266,9 @@ def roofline(bp_ms_per_launch, slices_per_launch, filter_ms_per_launch, smem_pea
     if os.path.exists(tpath):
         with open(tpath) as f:
             tr = json.load(f)
-        if not groups and "bp_fast_per_slice_bytes" in tr:
-            traffic = tr["bp_fast_per_slice_bytes"] * slices_per_launch
+        per = tr.get("bp_quad_per_slice_bytes" if groups else "bp_fast_per_slice_bytes")
+        if per:
+            traffic = per * slices_per_launch
     filt_bytes = 4.0 * N_ANGLES * WIDTH * 2 * slices_per_launch   # read + write rows
     hbm_peak = 6541.8
     mp = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -856,7 +857,7 @@ def run_ts(args, rank, world, local):
         "data": "synthetic (smooth absorption projections with 2 % seeded noise)",
         "config": {"workload": f"ts_add of {TS_PROJ} projections {TS_ROWS} x {TS_PIXELS} over "
                                f"+-30 deg into plane {plane}, centre {center}, RAMP, ABS",
-                   "fft_length": 8192},
+                   "fft_length": 6144},   # the lesser of 2^k and 3 2^k from 2 x 2560 on
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak,
                      "unit": "GB/s", "frac": round(achieved / hbm_peak, 4), "traffic": None,
                      "algorithmic_bytes_per_projection": bytes_per_proj},

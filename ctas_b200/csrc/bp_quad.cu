@@ -12,9 +12,9 @@
 //
 // What bounds it.  One slice at a time (bp_fast.cu) every update costs a 4-byte shared
 // load and an index: 4.1 instructions and 1.0 wavefronts per 32 updates, 1569 us per
-// slice of 1800 x 2560 (tile 15; 20.3 updates per clock and SM).  Here 2.2 instructions
-// and 0.62 wavefronts, 847 us (37.6): shared-memory wavefronts 68 % of their peak,
-// issue 64 %, FMA and integer pipes about 55 % each, none of which leaves much.
+// slice of 1800 x 2560 (tile 15; 20.3 updates per clock and SM).  Here 2.1 instructions
+// and 0.59 wavefronts, 847 us (37.6): shared-memory wavefronts 69 % of their peak,
+// issue 64 %, FMA and integer pipes 56 % each, none of which leaves much.
 //   * 16-byte loads of interleaved slices: 4 wavefronts serve 128 updates and the index
 //     arithmetic is shared, but alone they leave the wavefront bound where it was
 //     (1.0 per 32 updates): 1082 us.
@@ -30,6 +30,8 @@
 // The loop over projections is not unrolled: a pass is 130 instructions for each of 12
 // patterns and layouts, and twice that no longer stays in the instruction cache
 // (2398 us with 4 warps a CTA).  Half the pixels per thread, 24 warps an SM: 998 us.
+// QSmall keeps that register limit (three CTAs), but with 32 projections a stage its
+// windows leave room for two.
 // Linear interpolation (an extension, FP64-derived projection bases) uses the same
 // layouts and patterns with two loads per sample: 397 instead of 980 us per slice of
 // 900 x 1536, bound by registers (its samples, differences and fractions).

@@ -30,14 +30,17 @@
 // the epilogue's latency per tile.  Measured steps, with the same outputs bit for bit:
 //   * the issuing warp stays converged and one elected lane issues each MMA, so that
 //     descriptors and counters live in uniform registers: a single thread took about 100
-//     clocks per MMA to form them.  With outputs through TMA stores (drain32) and a
-//     wait's limit loaded only when its first try fails, the row form below went from
-//     270 to 187 us on 64 -> 64 at 2 x 1024 x 1024, 528 to 403 on 96 -> 32 at 2048 x 2048,
-//     207 to 144 on 32 -> 32 and 180 to 125 on 16 -> 32;
+//     clocks per MMA to form them;
+//   * outputs through TMA stores (drain32), and a wait's limit loaded only when its first
+//     try fails;
+//   * in the row form below the ring's segments as plain scalars (403 -> 312 us on 96 -> 32
+//     at 2048 x 2048).  Together the row form went from 270 to 169 us on 64 -> 64 at
+//     2 x 1024 x 1024, and at 2048 x 2048 from 528 to 312 on 96 -> 32, 207 to 129 on
+//     32 -> 32 and 180 to 115 on 16 -> 32;
 //   * resident weights, and all of tensor memory for the only CTA of an SM.
-// The tiled form with resident weights is faster still than the row form on 96 -> 32
-// (342 us) and 64 -> 64 (171), but adds a pixel's products in another order, which
-// changes the BF16 rounding of every layer after it.
+// The tiled form with resident weights runs 64 -> 64 in 171 us and 96 -> 32 in 342, no
+// faster than the row form, and it adds a pixel's products in another order, which
+// changes the BF16 rounding of every layer after it: a layer keeps its form.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -1046,8 +1049,8 @@ bool make_row_map(const ConvArgs &a, CUtensorMap *map) {
 // one kx.  Bound by the operands' shared-memory reads (6 KB, 48 clocks per MMA whose
 // math takes 32) and the issue of MMAs that short (70 clocks).  One tap per CTA, M = 128
 // output channels, read dy and x from L2 once per tap and was bound by that: 64 -> 64 at
-// 2 x 1024 x 1024 830 us, now 284; 32 -> 32 at 4 x 512 x 512 422 and 135, 192 -> 64 at
-// 2 x 512 x 512 448 and 218, 128 -> 128 at 4 x 256 x 256 129 and 95.
+// 2 x 1024 x 1024 830 us, now 285; 32 -> 32 at 4 x 512 x 512 422 and 135, 192 -> 64 at
+// 2 x 512 x 512 448 and 219, 128 -> 128 at 4 x 256 x 256 129 and 95.
 struct WgTcArgs {
   float *dw;
   int cin, cout;
