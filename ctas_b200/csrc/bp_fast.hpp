@@ -28,11 +28,12 @@ int bp_fast_search(const std::function<float(int)> &time_ms, bool all_variants);
 // own (15) 14.2.  Launches of few waves (up to eight 64 x 64 tiles per SM) are tuned for
 // their number of slices: three full-turn slices of 700 x 700 prefer tile 18, with which
 // five take 349 us, 222 with tile 14; eleven slices of 460 x 460 take 262 us with the
-// tile of ten, 199 with their own.
+// tile of ten, 199 with their own.  Trial centres of one sinogram come in varying numbers
+// from one search and share a choice.
 using TuneKey = std::tuple<int, int, int, int, int, int, int, bool, bool, int>;
 inline TuneKey bp_fast_tune_key(const BpLaunch &a, int device, bool rest, int sms = 148) {
   const int64_t tiles = (int64_t)((a.out_rows + 63) / 64) * ((a.out_cols + 63) / 64) * a.S;
-  const int few = tiles <= 8 * (int64_t)sms ? a.S : 0;
+  const int few = !a.centers && tiles <= 8 * (int64_t)sms ? a.S : 0;
   return TuneKey(device, a.W, a.N, a.store, a.interp, a.out_rows, a.out_cols, a.wide != 0, rest, few);
 }
 // Tile for this launch: `requested` if it is a valid id, else the

@@ -90,7 +90,8 @@ enum { CTAS_STORE_F32 = 0, CTAS_STORE_F16 = 1, CTAS_STORE_BF16 = 2 };
  * timeout path of the kernel: drain, error word, early return.) */
 #define CTAS_FLAG_TEST_TIMEOUT 0x200u
 /* Test aid: stacks of three or more slices go through the four-slice kernel
- * however small they are (it otherwise takes stacks that fill the device). */
+ * however small they are (it otherwise takes those that it is estimated to be
+ * faster for). */
 #define CTAS_FLAG_GROUPS 0x400u
 
 typedef struct ctas_fbp_opts {
@@ -118,9 +119,12 @@ typedef struct ctas_fbp_opts {
                              0 = auto                                              */
   int32_t tile;           /* staged backprojection tile id in
                              [0, ctas_fbp_tile_count()); -1 = autotune: the first
-                             launch of a shape times candidate tiles on one slice
-                             (this synchronises the stream once; do it before any
-                             stream capture); with struct_size below this field: -1 */
+                             launch of a shape, and of a small shape's slice count,
+                             times candidate tiles on some of its slices (this
+                             synchronises the stream once; under stream capture it
+                             is left out and a tile chosen for another count, else
+                             a fixed one, serves); with struct_size below this
+                             field: -1                                            */
   int32_t ring_box;       /* half width of the ring-artefact filter applied to every
                              sinogram before filtering (RingFilter::apply,
                              lct.cpp:295-327; the ct tool's -R); 0 = off          */

@@ -32,6 +32,10 @@ int main() {
     c.S = slices;
     return ctas::bp_fast_tune_key(c, 0, false, 148);
   };
+  const float centre = 0.f;
+  c.centers = &centre;
+  if (!(at(1) == at(33)) || !(at(8) == at(33))) return 31;
+  c.centers = nullptr;
   if (at(3) == at(5) || at(8) == at(9) || !(at(10) == at(40))) return 30;
   return 0;
 }
