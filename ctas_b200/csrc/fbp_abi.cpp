@@ -258,11 +258,14 @@ void init_streams(ctas_fbp *h) {
 
 // Whether stacks of this handle may go through the four-slice kernel: rows that serve
 // the index rule without branches (sines >= 0, or the reference's truncation on the wide
-// layout), and no tile asked for by id.  16-bit rows are expanded to float32 groups for it, a
+// layout), an output geometry whose rounding the kernel allows for, and no tile asked for
+// by id.  16-bit rows are expanded to float32 groups for it, a
 // bounded number at a time.
 bool quad_capable(const ctas_fbp *h) {
   return (h->sines_nonneg || h->wide) && h->geo_p > 0.f && h->geo_p <= 1.f && h->tile < 0 &&
-         h->tiles.in64 > 0 && !h->singles && !ctas::bp_fast_tile_forced();
+         h->tiles.in64 > 0 && !h->singles &&
+         ctas::quad_sharing_exact(h->W, h->out_rows, h->out_cols, h->geo_p) &&
+         !ctas::bp_fast_tile_forced();
 }
 
 ctas::QuadForm quad_form(const ctas_fbp *h) {
