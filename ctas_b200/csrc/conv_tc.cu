@@ -1045,19 +1045,20 @@ bool make_row_map(const ConvArgs &a, CUtensorMap *map) {
 // nine taps, into five tensor-memory accumulators.  The pixel blocks are split over
 // CTAs, which add their sums to dw.
 //
-// Where nine-tap CTAs would fill less than half of the device, a CTA has the taps of
-// one kx.  Bound by the operands' shared-memory reads (6 KB, 48 clocks per MMA whose
+// A CTA has the taps of one kx where those CTAs are all resident.  Bound by the operands' shared-memory reads (6 KB, 48 clocks per MMA whose
 // math takes 32) and the issue of MMAs that short (70 clocks).  One tap per CTA, M = 128
 // output channels, read dy and x from L2 once per tap and was bound by that: 64 -> 64 at
-// 2 x 1024 x 1024 830 us, now 285; 32 -> 32 at 4 x 512 x 512 422 and 135, 192 -> 64 at
-// 2 x 512 x 512 448 and 219, 128 -> 128 at 4 x 256 x 256 129 and 95.
+// 2 x 1024 x 1024 830 us, now 283; 32 -> 32 at 4 x 512 x 512 422 and 134, 192 -> 64 at
+// 2 x 512 x 512 448 and 216, 128 -> 128 at 4 x 256 x 256 129 and 88.  From 64 pixel blocks
+// on no layer is slower; images of 4096 pixels and less with 128 channels or more, one
+// block to a CTA, are by up to 1.7 us (256 -> 256 at 16 x 32 8.1 against 6.4).
 struct WgTcArgs {
   float *dw;
   int cin, cout;
   int bx, by;
   int64_t nblk;  // B * by * bx pixel blocks
   int ci_tiles, ksplit;
-  int n;         // MMA N: output channels of a tile, a multiple of 16
+  int n;         // MMA N: output channels of a tile, a multiple of 16, at most 64
   int *err;
 };
 
@@ -1066,6 +1067,20 @@ struct WgTcArgs {
 __device__ __forceinline__ uint64_t sdesc_mn128(uint32_t addr, uint32_t lbo) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+// 4 x 4 transpose among four neighbouring lanes: lane r of them gives v[c] as element
+// (r, c) and has element (c, r) as v[c] after.
+__device__ __forceinline__ void transpose4(float (&v)[4], int lane) {
+  const bool r0 = lane & 1, r1 = lane & 2;
+  float t = __shfl_xor_sync(0xffffffffu, r0 ? v[0] : v[1], 1);
+  (r0 ? v[0] : v[1]) = t;
+  t = __shfl_xor_sync(0xffffffffu, r0 ? v[2] : v[3], 1);
+  (r0 ? v[2] : v[3]) = t;
+  t = __shfl_xor_sync(0xffffffffu, r1 ? v[0] : v[2], 2);
+  (r1 ? v[0] : v[2]) = t;
+  t = __shfl_xor_sync(0xffffffffu, r1 ? v[1] : v[3], 2);
+  (r1 ? v[1] : v[3]) = t;
 }
 
 constexpr int kWgRow = 16 * 128;          // 16 pixels x 64 channels x 2 B
@@ -1158,7 +1173,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         mbar_expect_tx(&full[2 * stage], (uint32_t)((G == 1 ? 2 : 1) * kWgBox + 8 * kWgRow));
         if (G == 1) mbar_expect_tx(&full[2 * stage + 1], (uint32_t)kWgBox);
         if (!stall) {
-          tma_load_4d(sd, &dymap, cot * 64, tx * 16, ty * 8, b, &full[2 * stage]);
+          tma_load_4d(sd, &dymap, cot * a.n, tx * 16, ty * 8, b, &full[2 * stage]);
           box(0, &full[2 * stage]);
           if (G == 1) {
             box(1, &full[2 * stage]);
@@ -1248,23 +1263,34 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     if (ok && b1 > b0 && !__shfl_sync(0xffffffffu, *s_abort, 0)) {
       tc_fence_after();
-      // row (half, ci) of every accumulator: consecutive lanes add consecutive input
-      // channels
-      const int half = row >> 6, ci = cit * 64 + (row & 63);
+      // row (half, ci) of every accumulator.  Four lanes exchange 4 x 4 blocks, so that each
+      // adds 16 bytes: four input channels of one output channel, eight such lanes side
+      // by side (dw and rows of 16 channels and more are 16-byte aligned).  4-byte adds
+      // took 17.1 us for one pixel block and 64 x 64 channels in one CTA, these 11.6.
+      const int half = row >> 6, ci = cit * 64 + (row & 60);
 #pragma unroll 1
       for (int acc = 0; acc < C::kAcc; acc++) {
         const int tap = C::tap(acc, half, kx0);
 #pragma unroll 1
-        for (int c0 = 0; c0 < a.n; c0 += 16) {
-          uint32_t rr[16];
-          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(64 * acc + c0), rr);
+        for (int c0 = 0; c0 < a.n; c0 += 32) {
+          // two 16-column loads in flight; the second is not used by a tile of 16 or 48
+          uint32_t rr[2][16];
+          const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(64 * acc + c0);
+          tmem_ld16(taddr, rr[0]);
+          tmem_ld16(taddr + 16u, rr[1]);
           tmem_wait_ld();
-          if (tap >= 0 && ci < a.cin) {
+          float *o = a.dw + ((int64_t)(cot * a.n + c0 + (lane & 3)) * 9 + tap) * a.cin + ci;
+          const int left = tap >= 0 && ci < a.cin
+                               ? min(a.n - c0, a.cout - cot * a.n - c0) - (lane & 3) : 0;
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-              const int co = cot * 64 + c0 + j;
-              if (co < a.cout) atomicAdd(a.dw + ((int64_t)co * 9 + tap) * a.cin + ci, __uint_as_float(rr[j]));
-            }
+          for (int c = 0; c < 32; c += 4) {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = __uint_as_float(rr[c >> 4][(c & 15) + j]);
+            transpose4(v, lane);
+            if (c < left)
+              atomicAdd(reinterpret_cast<float4 *>(o + (int64_t)c * 9 * a.cin),
+                        make_float4(v[0], v[1], v[2], v[3]));
           }
         }
       }
@@ -1415,9 +1441,8 @@ cudaError_t launch_conv3x3_wgrad_tc(const WgradArgs &a, cudaStream_t st) {
   w.bx = a.W / 16;
   w.by = a.H / 8;
   w.nblk = (int64_t)a.B * w.by * w.bx;
-  w.n = std::min(64, a.cout);
   w.ci_tiles = (a.cin + 63) / 64;
-  const int tiles = w.ci_tiles * ((a.cout + 63) / 64);
+  int tiles = w.ci_tiles * ((a.cout + 63) / 64);
   // K splits: as many as fill the device twice with tiles of 128 output channels x 64 or
   // 128 input channels x one tap.  The tensor cores' accumulation truncates, so the
   // split decides the result to 1e-4 of it, and stays where it was when a CTA had one
@@ -1426,9 +1451,16 @@ cudaError_t launch_conv3x3_wgrad_tc(const WgradArgs &a, cudaStream_t st) {
   w.ksplit = (int)std::max<int64_t>(1, std::min<int64_t>(w.nblk, (2LL * sm_count() + cols - 1) / cols));
   cudaError_t e = err_word(&w.err);
   if (e != cudaSuccess) return e;
-  // a CTA per kx where the nine-tap CTAs would leave most of the device idle
-  return 2 * tiles * w.ksplit <= sm_count() ? launch_wgrad<3>(dymap, xmap, w, tiles, st)
-                                            : launch_wgrad<1>(dymap, xmap, w, tiles, st);
+  // A CTA per kx where all of them are resident at once, two to an SM (64 -> 128 at
+  // 64 x 64, 64 nine-tap CTAs: 8.1 against 11.7 us; 128 -> 128 at 128 x 128, 132: 17.8 and
+  // 15.9), and 32 output channels each where those are still resident and have few pixel
+  // blocks, so that adding them up is most of the time (64 -> 64 at 32 x 32 5.4 against
+  // 6.7 us, at 128 x 128 8.6 both ways).
+  const bool three = 3 * tiles * w.ksplit <= 2 * sm_count();
+  const bool half = three && 6 * tiles * w.ksplit <= 2 * sm_count() && w.nblk <= 4 * w.ksplit;
+  w.n = std::min(half ? 32 : 64, a.cout);
+  tiles = w.ci_tiles * ((a.cout + w.n - 1) / w.n);
+  return three ? launch_wgrad<3>(dymap, xmap, w, tiles, st) : launch_wgrad<1>(dymap, xmap, w, tiles, st);
 }
 
 int conv_tc_error() {

@@ -1,18 +1,19 @@
-"""The weight gradient's nine-tap form (all nine taps of a tile in one CTA), which layers
-of 128 and more channels take: values against torch, and its bounded waits."""
+"""The weight gradient's forms: all nine taps of a tile in one CTA, which layers of 128 and
+more channels take, and those of one kx with 64 or 32 output channels: values against
+torch, and the bounded waits of the first."""
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
 def _nine_taps(cin, cout, B, H, W):
-    """The dispatch's rule: unless the nine-tap CTAs would fill less than half the device."""
+    """The dispatch's rule: unless CTAs of one kx are all resident, two to an SM."""
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     tiles = -(-cin // 64) * -(-cout // 64)
     cols = 9 * -(-cout // 128) * (-(-cin // 128) if cin > 64 else 1)
     split = max(1, min(B * (H // 8) * (W // 16), (2 * sms + cols - 1) // cols))
-    return 2 * tiles * split > sms
+    return 3 * tiles * split > 2 * sms
 
 
 def _data(cin, cout, B, H, W):
@@ -43,6 +44,26 @@ def test_nine_tap_gradient_matches_torch(cin, cout, B, H, W):
     ref = ref.permute(0, 2, 3, 1).reshape(cout, 9, cin)
     torch.cuda.synchronize()
     assert float((dw - 2.0 - ref).abs().max()) <= 1e-3 * float(ref.abs().max())
+
+
+# one kx: 32 output channels a CTA (few blocks; 48, 80 and 112 leave partial tiles, 16 is
+# below one), 64 where there are more blocks or CTAs
+@pytest.mark.parametrize("cin,cout,B,H,W", [
+    (16, 16, 1, 8, 16), (32, 48, 1, 16, 32), (64, 80, 1, 16, 32), (128, 112, 1, 8, 32),
+    (48, 32, 2, 32, 32), (64, 64, 1, 32, 32), (64, 64, 2, 64, 256), (32, 64, 4, 64, 128),
+    (192, 64, 1, 32, 32), (64, 128, 2, 64, 64), (80, 48, 1, 64, 128), (256, 256, 1, 8, 16)])
+def test_one_kx_gradient_matches_torch(cin, cout, B, H, W):
+    import torch
+    from ctas_b200 import learned
+    assert not _nine_taps(cin, cout, B, H, W)
+    x, dy = _data(cin, cout, B, H, W)
+    dw = torch.full((cout, 9, cin), -1.0, device="cuda")
+    learned.conv3x3_wgrad(x, dy, dw)
+    ref = torch.nn.grad.conv2d_weight(x.double().permute(0, 3, 1, 2), (cout, cin, 3, 3),
+                                      dy.double().permute(0, 3, 1, 2), padding=1)
+    ref = ref.permute(0, 2, 3, 1).reshape(cout, 9, cin)
+    torch.cuda.synchronize()
+    assert float((dw + 1.0 - ref).abs().max()) <= 1e-3 * float(ref.abs().max())
 
 
 def test_channel_slices():
