@@ -713,11 +713,15 @@ constexpr int kRowPx = 130;                    // 128 output pixels + 2 halo
 constexpr int kRowChunkBytes = 17 * 1024;      // 130 x 128 B, padded to the 1 KB atom
 constexpr int kRowMaxSlots = 8;
 constexpr int kMaxAcc = 8;
-// staging buffers per epilogue warp: one for 128 input channels, whose 128 -> 32 layer
-// fits shared memory only so (weights, four input rows and 8 KB of staging: 224,536 of
-// 232,448 bytes)
-__host__ __device__ constexpr int row_bufs(int cin) { return cin == 128 ? 1 : 2; }
-__host__ __device__ constexpr int row_out(int cin) { return 4 * row_bufs(cin) * kOutBytes; }
+// Bias of all output channels, barriers and two words: behind the staging buffers, or with
+// one buffer per epilogue warp in the padding of the first row buffer, where 64 -> 32 and
+// 32 -> 64 so fit twice into an SM (115,712 bytes each): at 2 x 1024 x 1024 96 us instead
+// of 139, which one CTA took, and 94 instead of 131.
+constexpr int kRowMaxCout = 64;
+constexpr int kRowTail = 4 * kRowMaxCout + (2 * kRowMaxSlots + 2 * kMaxAcc + 1) * 8 + 8;
+constexpr int kRowPad = kRowPx * 128;          // start of that padding
+static_assert(kRowPad % 16 == 0 && kRowPad + kRowTail <= kRowChunkBytes,
+              "bias and barriers in the padding of a row buffer");
 
 struct RowArgs {
   const bf16 *mask;
@@ -758,7 +762,8 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-template <int CIN>
+// BUFS: staging buffers per epilogue warp, 1 or 2
+template <int CIN, int BUFS>
 __global__ void __launch_bounds__(kThreads, 1)
     conv_row_kernel(const __grid_constant__ CUtensorMap amap,
                     const __grid_constant__ CUtensorMap ymap, RowArgs a) {
@@ -768,8 +773,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t *slots = base;                                   // input-row ring (1 KB atoms)
   uint8_t *wsm = base + a.nslots * a.slot_bytes;           // weights
   uint8_t *outs = wsm + a.wbytes;                          // output staging
-  float *s_bias = reinterpret_cast<float *>(outs + row_out(CIN));
-  uint64_t *row_full = reinterpret_cast<uint64_t *>(s_bias + kMaxCout);
+  float *s_bias = reinterpret_cast<float *>(BUFS == 1 ? base + kRowPad : outs + 4 * BUFS * kOutBytes);
+  uint64_t *row_full = reinterpret_cast<uint64_t *>(s_bias + kRowMaxCout);
   uint64_t *row_empty = row_full + kRowMaxSlots;
   uint64_t *acc_full = row_empty + kRowMaxSlots;  // [kMaxAcc]
   uint64_t *acc_empty = acc_full + kMaxAcc;
@@ -979,9 +984,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * cout);
 #pragma unroll 1
         for (int c0 = 0; c0 < cout; c0 += 32, turn ^= 1) {
-          constexpr int kBufs = row_bufs(CIN);
-          uint8_t *so = outs + (kBufs == 2 ? 2 * q + turn : q) * kOutBytes;
-          drain32<kBufs - 1>(taddr + (uint32_t)c0, s_bias + c0, mp ? mp + c0 : nullptr, a.relu, so, lane);
+          uint8_t *so = outs + (BUFS == 2 ? 2 * q + turn : q) * kOutBytes;
+          drain32<BUFS - 1>(taddr + (uint32_t)c0, s_bias + c0, mp ? mp + c0 : nullptr, a.relu, so, lane);
           if (lane == 0) tma_store_4d(&ymap, so, c0, sx * 128 + q * 32, y, b);
         }
         tc_fence_before();
@@ -1004,17 +1008,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                  : "memory");
 }
 
-// bias, barriers, slack
-constexpr int kRowSmemFixed = 4 * kMaxCout + (2 * kRowMaxSlots + 2 * kMaxAcc + 1) * 8 + 16 + 1024;
 constexpr int kRowSmemMax = 232448, kRowSmemHalf = 233472 / 2 - 1024;
 
 // resident weights of the row form: 9 taps x cout rows x cin channels
 int row_wbytes(const ConvArgs &a) { return 9 * a.cin * a.cout * 2; }
 
-// shared memory of the row form for `slots` input-row buffers
-int row_smem(const ConvArgs &a, int slots) {
-  return row_wbytes(a) + slots * ((a.cin + 63) / 64) * kRowChunkBytes + row_out(a.cin) +
-         kRowSmemFixed;
+// shared memory of the row form for `slots` input-row buffers and `bufs` staging buffers
+// per epilogue warp, with 1 KB to align them
+int row_smem(const ConvArgs &a, int slots, int bufs) {
+  return row_wbytes(a) + slots * ((a.cin + 63) / 64) * kRowChunkBytes + 4 * bufs * kOutBytes +
+         (bufs == 1 ? 0 : kRowTail) + 1024;
+}
+// One staging buffer where that puts a second CTA on the SM, or the layer on it at all.
+int row_bufs(const ConvArgs &a) {
+  const int most = row_smem(a, 4, 1) <= kRowSmemHalf ? kRowSmemHalf : kRowSmemMax;
+  return row_smem(a, 4, 2) <= most ? 2 : 1;  // 1: 32 -> 64 and 64 -> 32
 }
 
 bool make_row_map(const ConvArgs &a, CUtensorMap *map) {
@@ -1350,7 +1358,7 @@ bool conv_row_ok(const ConvArgs &a) {
   return conv_tc_ok(a) && a.W % 128 == 0 &&
          (a.cin == 16 || a.cin == 32 || a.cin == 64 || a.cin == 96 || a.cin == 128) &&
          a.cout % 32 == 0 &&
-         a.cout <= 64 && row_wbytes(a) <= 112 * 1024 && row_smem(a, 4) <= kRowSmemMax;
+         a.cout <= kRowMaxCout && row_wbytes(a) <= 112 * 1024 && row_smem(a, 4, 1) <= kRowSmemMax;
 }
 
 cudaError_t launch_conv3x3_row(const ConvArgs &a, cudaStream_t st) {
@@ -1369,24 +1377,25 @@ cudaError_t launch_conv3x3_row(const ConvArgs &a, cudaStream_t st) {
   r.H = a.H;
   r.W = a.W;
   // half of tensor memory for each of two CTAs per SM, all of it for one
-  r.cols = row_smem(a, 4) <= kRowSmemHalf ? 256u : 512u;
+  const int bufs = row_bufs(a);
+  r.cols = row_smem(a, 4, bufs) <= kRowSmemHalf ? 256u : 512u;
   r.nacc = std::min<int>(kMaxAcc, (int)r.cols / a.cout);
   r.wbytes = row_wbytes(a);
   r.slot_bytes = ((a.cin + 63) / 64) * kRowChunkBytes;
   // two CTAs per SM where four input rows fit beside the weights, else one
   const int most = r.cols == 256u ? kRowSmemHalf : kRowSmemMax;
   int slots = kRowMaxSlots;
-  while (slots > 4 && row_smem(a, slots) > most) slots--;
+  while (slots > 4 && row_smem(a, slots, bufs) > most) slots--;
   r.nslots = slots;
   cudaError_t e = err_word(&r.err);
   if (e != cudaSuccess) return e;
   const int per_sm = 512 / (int)r.cols;
-  const int smem = std::max(row_smem(a, slots), 232448 / (per_sm + 1) + 1024);
-  auto kern = a.cin == 16   ? conv_row_kernel<16>
-              : a.cin == 32 ? conv_row_kernel<32>
-              : a.cin == 64 ? conv_row_kernel<64>
-              : a.cin == 96 ? conv_row_kernel<96>
-                            : conv_row_kernel<128>;
+  const int smem = std::max(row_smem(a, slots, bufs), 232448 / (per_sm + 1) + 1024);
+  auto kern = a.cin == 16   ? conv_row_kernel<16, 2>
+              : a.cin == 32 ? (bufs == 1 ? conv_row_kernel<32, 1> : conv_row_kernel<32, 2>)
+              : a.cin == 64 ? (bufs == 1 ? conv_row_kernel<64, 1> : conv_row_kernel<64, 2>)
+              : a.cin == 96 ? conv_row_kernel<96, 2>
+                            : conv_row_kernel<128, 2>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
