@@ -15,7 +15,8 @@
 //      keeps every operand start on a swizzle-atom boundary;
 //   B: the weights viewed as a 2-D array [cout][9 cin]; three NT x CK boxes per
 //      (kx, chunk), one per ky tap, placed one after another -- loaded once and kept
-//      where all of them fit beside the input boxes, else with each input box.
+//      where all of them fit beside the input boxes and a CTA has several tiles, else
+//      with each input box.
 //
 // Persistent warp-specialised CTA (192 threads): warp 0 issues the TMA loads
 // into a ring of stages, warp 1 issues the MMAs (K = 16 each) and releases each
@@ -673,13 +674,17 @@ cudaError_t launch_cfg(const ConvArgs &a, cudaStream_t st) {
 
 // Whether the weights of all nine taps fit beside three input boxes (64 -> 128, 128 -> 64
 // and the layers below on rows that the row form does not take): the CTAs then read
-// them once instead of per tile.  64 -> 128 at 2 x 512 x 512 91 -> 70 us.
-template <int CK, int NT> bool resident_fits(const ConvArgs &a) {
-  return a.cout == NT && TcCfg<CK, NT, 0>::smem(3, a.cin / CK) <= 232448;
+// them once instead of per tile.  64 -> 128 at 2 x 512 x 512 91 -> 70 us.  From more than
+// two tiles per SM on: a CTA with one tile waits for all weights before its first MMA
+// (32 -> 32 at 64 x 64 5.6 us resident and 5.3 with the input boxes, at 2 x 128 x 144 6.2
+// and 5.9, at 2 x 256 x 208 8.8 and 9.3).
+template <int CK, int NT> bool resident_pays(const ConvArgs &a) {
+  return a.cout == NT && TcCfg<CK, NT, 0>::smem(3, a.cin / CK) <= 232448 &&
+         (int64_t)a.B * (a.H / 8) * (a.W / 16) > 2 * sm_count();
 }
 
 template <int CK, int NT> cudaError_t launch_ck_nt(const ConvArgs &a, cudaStream_t st) {
-  if (resident_fits<CK, NT>(a)) return launch_cfg<CK, NT, 0>(a, st);
+  if (resident_pays<CK, NT>(a)) return launch_cfg<CK, NT, 0>(a, st);
   constexpr int kStage = 160 * CK * 2 + 3 * NT * CK * 2;
   constexpr int kSt = (96 * 1024) / kStage < 2 ? 2 : (96 * 1024) / kStage > 6 ? 6 : (96 * 1024) / kStage;
   return launch_cfg<CK, NT, kSt>(a, st);
