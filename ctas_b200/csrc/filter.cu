@@ -296,7 +296,9 @@ __device__ __forceinline__ float pow2_scale(float mx) {
 // Filters rows 2*pair and 2*pair+1 of slice sl.  Called by every thread of
 // the CTA with the CTA's dynamic shared memory (P + P/16 float2).  THREE: P is 3 times a
 // power of two, its first radix 3 (every later stride is a power of two).
-template <typename T, bool THREE = false>
+// GROUP: the interleaved layout and the dense copy are served; the plain form carries
+// neither (with both decided at run time it ran 2 to 5 % slower).
+template <typename T, bool THREE = false, bool GROUP = false>
 __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int sl) {
   extern __shared__ float2 sm[];
   __shared__ float red[2][kFftThreads / 32];
@@ -328,7 +330,7 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
   // the kernel's time: one of evenly spaced samples is wrong for a row of their period.
   float2 mean = make_float2(0.f, 0.f);
   if (THREE && a.periodic) {
-#pragma unroll 4
+#pragma unroll 8
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
       mean.x += abs_mode ? deabs(x0[c], mm) : x0[c];
       if (has1) mean.y += abs_mode ? deabs(x1[c], mm) : x1[c];
@@ -393,13 +395,14 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
   // row-wide epilogue (REF running sum, reduced-precision scale) needs them
   const bool direct = ns >= 2 && a.contrast != 1 && a.store == 0;
   // es: elements between samples of a row, ep: between rows
-  const int es = a.quad ? kQuadSlices : 1;
+  const bool quad = GROUP && a.quad;
+  const int es = quad ? kQuadSlices : 1;
   const int64_t ep = (int64_t)es * a.Wp;
-  T *q0 = reinterpret_cast<T *>(a.q) + (a.quad ? (sl / kQuadSlices) * a.q_slice_stride + sl % kQuadSlices
-                                               : sl * a.q_slice_stride) +
+  T *q0 = reinterpret_cast<T *>(a.q) + (quad ? (sl / kQuadSlices) * a.q_slice_stride + sl % kQuadSlices
+                                             : sl * a.q_slice_stride) +
           (int64_t)r0 * ep + (a.off ? a.off : kRowOff) * es;
   T *q1 = q0 + ep;
-  float *d0 = a.dense ? a.dense + ((int64_t)sl * N + r0) * W : nullptr;
+  float *d0 = GROUP && a.dense ? a.dense + ((int64_t)sl * N + r0) * W : nullptr;
 
   if (ns >= 2) {
     const int R = a.radix[0];
@@ -571,7 +574,12 @@ __global__ void __launch_bounds__(kFftThreads) filter_three_kernel(FilterLaunch 
 // their blocks for one row pair are neighbours and the sectors fill in L2.
 __global__ void __launch_bounds__(kFftThreads) filter_quad_kernel(FilterLaunch a) {
   const int sl = kQuadSlices * blockIdx.y + (blockIdx.x & (kQuadSlices - 1));
-  if (sl < a.S) filter_pair<float>(a, blockIdx.x / kQuadSlices, sl);
+  if (sl < a.S) filter_pair<float, false, true>(a, blockIdx.x / kQuadSlices, sl);
+}
+
+// Slices of the padded layout that are stored densely too.
+__global__ void __launch_bounds__(kFftThreads) filter_dense_kernel(FilterLaunch a) {
+  filter_pair<float, false, true>(a, blockIdx.x, blockIdx.y);
 }
 
 // Uneven batch: one launch over the row pairs of every sinogram; jobs[k]
@@ -795,15 +803,19 @@ cudaError_t launch_filter_three(const FilterLaunch &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_filter_quad(const FilterLaunch &a, cudaStream_t st) {
+// quad: whole groups of the interleaved layout, else slices with a dense copy
+cudaError_t launch_filter_group(const FilterLaunch &a, cudaStream_t st) {
+  auto kern = a.quad ? filter_quad_kernel : filter_dense_kernel;
   const size_t smem = sizeof(float2) * (size_t)(a.P + a.P / 16);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        filter_quad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  const dim3 grid(kQuadSlices * ((a.N + 1) / 2), (a.S + kQuadSlices - 1) / kQuadSlices);
-  filter_quad_kernel<<<grid, kFftThreads, smem, st>>>(a);
+  const int pairs = (a.N + 1) / 2;
+  const dim3 grid = a.quad ? dim3(kQuadSlices * pairs, (a.S + kQuadSlices - 1) / kQuadSlices)
+                           : dim3(pairs, a.S);
+  kern<<<grid, kFftThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -848,8 +860,8 @@ cudaError_t launch_expand_quad(const void *q, int64_t q_slice_stride, const floa
 cudaError_t launch_filter(const FilterLaunch &a, cudaStream_t st) {
   if (a.contrast != 3 && a.nradix > 0 && a.radix[0] == 3)
     return launch_filter_three(a, st);
-  if (a.quad && a.store != 0) return cudaErrorInvalidValue;
-  if (a.quad && a.contrast != 3) return launch_filter_quad(a, st);
+  if ((a.quad || a.dense) && a.store != 0) return cudaErrorInvalidValue;
+  if ((a.quad || a.dense) && a.contrast != 3) return launch_filter_group(a, st);
   if (a.store == 1) return launch_filter_t<__half>(a, st);
   if (a.store == 2) return launch_filter_t<__nv_bfloat16>(a, st);
   return launch_filter_t<float>(a, st);
