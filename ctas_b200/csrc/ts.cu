@@ -9,10 +9,11 @@
 // "periodic" mode) and multiplied by G_P = DFT_P(h), h the kernel g laid symmetrically
 // about 0 (|d| <= n/2; for even n the d = n/2 tap is split between +-n/2).  For outputs
 // n/2 .. 3n/2 - 1 every tap reads inside the two periods, so the result is the circular
-// convolution up to float rounding.  P is the lesser of 2^k and 3 2^k: the filter is
-// bound by its passes over P elements in shared memory (6144 instead of 8192 for rows
-// of 2560).  5 2^k (5120 there) ran in 0.94 ms where 3 2^k takes 1.16 ms on
-// 31 x 1024 x 2560, but its rounding error on rows whose mean is small against their
+// convolution up to float rounding.  P is the next 2^k, or 3 2^k where that is less and
+// shortens the call (three_pays): the filter is bound by its passes over P elements in
+// shared memory (6144 instead of 8192 for rows of 2560).  The choice does not depend on
+// the number of images, so that a batch equals single calls.  5 2^k (5120 there) ran in
+// 0.94 ms where 3 2^k takes 1.16 ms on 31 x 1024 x 2560, but its rounding error on rows whose mean is small against their
 // range is up to 10 % above that of 2^k, in every form of the twiddles and the mean
 // (filter.cu), and is not used.
 //
@@ -170,6 +171,15 @@ std::vector<double> ts_window(const std::vector<float> &fwin, int64_t n, int64_t
   return G;
 }
 
+// Whether the transform of 3 2^k, which costs a pass for the rows' mean and longer
+// twiddle tables, is the faster one: where 2^k is 8192 or 16384 and the row pairs of one
+// image more than its CTAs that the device holds (three and one to an SM).  9 images of
+// 1024 x 1500 take 183 us at 4096 and 198 at 3072; one of 256 x 2560 39 us at 8192 and 42
+// at 6144, of 1024 x 2560 78 and 65, 31 of 1024 x 6000 5.8 and 3.6 ms.
+bool three_pays(int64_t P, int64_t rows, int sms) {
+  return P >= 8192 && (rows + 1) / 2 > (int64_t)sms * (P == 8192 ? 3 : 1);
+}
+
 void ts_create(ctas_ts *h, int64_t rows, int64_t pixels, int32_t ftype, float fparam,
                int32_t contrast, int32_t device) {
   if (rows < 1 || pixels < 2)
@@ -189,9 +199,10 @@ void ts_create(ctas_ts *h, int64_t rows, int64_t pixels, int32_t ftype, float fp
   h->P = ctas::padded_width(pixels);
   if (h->P > 16384)  // the row-pair FFT lives in shared memory
     ctas::fail(CTAS_E_UNSUPPORTED, "tomosynthesis: rows wider than 8192 pixels are not supported");
-  int64_t three = 48;  // 3 2^k of at least two stages behind the radix of 3
-  while (three < 2 * pixels) three *= 2;
-  h->P = std::min(h->P, three);
+  int sms = 148;
+  cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+  const int64_t three = h->P / 4 * 3;
+  if (three >= 2 * pixels && three_pays(h->P, rows, sms)) h->P = three;
   h->Wp = ctas::padded_pitch(pixels);
   // ts_add filters for every contrast; ABS adds -log, REF the running sum
   h->contrast = contrast == CTAS_FLT ? CTAS_PHS : contrast;

@@ -137,19 +137,60 @@ def test_restatement_filters():
             assert _error(_filter_pow2(x, fwin), _exact(x, fwin)) < 1e-4, (n, kind)
 
 
-# 600, 2560: the filter's 5 2^k lengths of earlier; 768, 1536, 3072: the transform full
+def _tall(n):
+    """Rows of an image that takes the transform of 3 2^k (ts.cu, three_pays)."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return 2 * sms * (3 if n <= 4096 else 1) + 3
+
+
+# 3072, 6144: the transform full; 2049, 4097: the shortest rows of each length
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", KINDS)
-@pytest.mark.parametrize("n", [600, 768, 1025, 1200, 1536, 2560, 3072])
+@pytest.mark.parametrize("n", [2049, 2560, 3072, 4097, 6144])
 def test_error_not_above_power_of_two(n, kind):
-    """Over 64 rows, whose errors scatter by a few per cent: at most 1.03 times."""
+    """Over 64 rows of a tall image, whose errors scatter by a few per cent: at most 1.03
+    times."""
     from ctas_b200 import ct, ts
     import torch
     fl = ct.Filter("RAMP")
     fwin = O.filter_fill_plain(fl.filter(), 0.0, n)
     x = _rows(kind, n, 64)
-    d = torch.from_numpy(x).cuda()
-    with ts.TS(x.shape, fl, ct.Contrast.PHS) as t:
+    d = torch.zeros((_tall(n), n), device="cuda")
+    d[:64] = torch.from_numpy(x).cuda()
+    with ts.TS(tuple(d.shape), fl, ct.Contrast.PHS) as t:
         t.add_batch_dev(d[None], np.zeros(1, f32), torch.zeros_like(d), 0.0, 0)
     want = _exact(x, fwin)
-    assert _error(d.cpu().numpy(), want) <= 1.03 * _error(_filter_pow2(x, fwin), want)
+    assert _error(d[:64].cpu().numpy(), want) <= 1.03 * _error(_filter_pow2(x, fwin), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2049, 2560, 3072, 4098, 6144])
+@pytest.mark.parametrize("cn", ["PHS", "ABS", "REF"])
+def test_tall_images_vs_oracle(n, cn):
+    """First and last rows of a tall image with an odd number of rows, filtered and added,
+    against the oracle's exact circular convolution: the bounds of the other widths (1e-5
+    of the filtered rows' range, 1e-4 with the running sum of refraction contrast); two
+    calls and a batch of two give the same bits."""
+    import torch
+    from ctas_b200 import ct, ts
+    rows, g, x = _tall(n), np.random.default_rng(n), np.linspace(-1, 1, n)
+    pick = [0, 1, 2, rows - 2, rows - 1]
+    proj = (0.6 + 0.3 * np.exp(-(x / 0.3) ** 2) + 0.02 * g.standard_normal((rows, n))).astype(f32)
+    res = g.standard_normal((rows, n)).astype(f32)
+    contrast, fl = getattr(ct.Contrast, cn), ct.Filter("RAMP")
+    want_p, want_r = O.ts_add(proj[pick], res[pick], fl.filter(), 0.0, 1.5, contrast, 0.3, 5)
+    with ts.TS((rows, n), fl, contrast) as t:
+        p, r = proj.copy(), res.copy()
+        t.add(p, r, 1.5, 0.3, 5)
+        one, two = torch.from_numpy(res).cuda(), torch.from_numpy(res).cuda()
+        d = torch.from_numpy(np.stack([proj, proj[::-1].copy()])).cuda()
+        angles = np.array([0.3, -0.2], f32)
+        for k in (0, 1):
+            t.add_batch_dev(d[k:k + 1].clone(), angles[k:k + 1], one, 1.5, 5)
+        t.add_batch_dev(d, angles, two, 1.5, 5)
+        torch.cuda.synchronize()
+    assert torch.equal(one.view(torch.int32), two.view(torch.int32))
+    tol = (1e-4 if cn == "REF" else 1e-5) * float(np.ptp(want_p))
+    assert float(np.abs(p[pick] - want_p).max()) <= tol
+    assert float(np.abs(r[pick] - want_r).max()) <= tol + 4 * float(np.spacing(np.abs(want_r).max()))
