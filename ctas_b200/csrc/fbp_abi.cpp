@@ -685,33 +685,61 @@ std::vector<int64_t> chunk_plan(int64_t n, int64_t C, int64_t unit) {
   return plan;
 }
 
+// Estimated time of the filters and backprojections of a chunk of S slices, us: filters at
+// their measured rate (90 us per 1800 x 2560 slice at 8192 points).
+double chunk_us(const ctas_fbp *h, int64_t S) {
+  const double filter = h->contrast == CTAS_FLT ? 0.0 : 4.7e-7 * h->N * h->P * std::log2((double)h->P);
+  return 10.0 + S * filter +
+         h->N / 720.0 * ctas::stack_us(quad_form(h), h->tiles, S, quad_count(h, S), h->sms, 1.08);
+}
+
+constexpr double kPinnedBytesUs = 50e3, kPageableBytesUs = 12e3;  // copies, each way
+
 // Estimated time of the host stack call's pipeline over `plan`, us: upload, compute and
 // download run beside one another, and a chunk's upload waits for the download two
-// chunks before it, whose buffers it takes.  Copies at 50 GB/s each way from and to
-// pinned memory and 12 GB/s else, where they return only when they are done; filters at
-// their measured rate (90 us per 1800 x 2560 slice at 8192 points).
+// chunks before it, whose buffers it takes.  Copies from and to pageable memory return
+// only when they are done.
 double plan_us(const ctas_fbp *h, const std::vector<int64_t> &plan, bool wb, bool pinned) {
-  const double bytes_us = pinned ? 50e3 : 12e3;
+  const double bytes_us = pinned ? kPinnedBytesUs : kPageableBytesUs;
   const double NW = (double)h->N * h->W, OO = (double)h->out_rows * h->out_cols;
-  const double filter = h->contrast == CTAS_FLT ? 0.0 : 4.7e-7 * h->N * h->P * std::log2((double)h->P);
   double in = 0, done = 0, out = 0, out_before = 0;
   for (const int64_t S : plan) {
     in = std::max(in, pinned ? out_before : out) + 4.0 * S * NW / bytes_us;
-    done = std::max(done, in) + 10.0 + S * filter +
-           h->N / 720.0 * ctas::stack_us(quad_form(h), h->tiles, S, quad_count(h, S), h->sms, 1.08);
+    done = std::max(done, in) + chunk_us(h, S);
     out_before = out;
     out = std::max(out, done) + 4.0 * S * (OO + (wb ? NW : 0.0)) / bytes_us;
   }
   return out;
 }
 
-// Chunks of the host calls.  Groups of four need chunks of at least four slices, whose
-// copies overlap less: four slices of 180 x 4096, bound by their copies, took 6.7 ms in
-// one chunk and 5.5 ms in four.  The faster of both is taken, by estimate.
+// The same for the volume call in chunks of C slices: its callbacks fill and empty three
+// pinned buffers each way beside the copies, in their own threads, and are taken to move
+// as many bytes as a copy of pageable memory.
+double volume_us(const ctas_fbp *h, int64_t n, int64_t C, int64_t sample_bytes) {
+  const double row = 4.0 * h->N * h->W, img = (double)sample_bytes * h->out_rows * h->out_cols;
+  double read = 0, done = 0, in[3] = {}, out[3] = {}, write[3] = {};  // of the last chunks
+  for (int64_t k = 0, s = 0; s < n; k++, s += C) {
+    const double S = (double)std::min(C, n - s);
+    double &i = in[k % 3], &o = out[k % 3], &w = write[k % 3];
+    const double i1 = in[(k + 2) % 3], o1 = out[(k + 2) % 3], o2 = out[(k + 1) % 3];
+    read = std::max(read, i) + S * row / kPageableBytesUs;
+    i = std::max({read, i1, o2}) + S * row / kPinnedBytesUs;
+    done = std::max(done, i) + chunk_us(h, (int64_t)S);
+    o = std::max({done, o1, w}) + S * img / kPinnedBytesUs;
+    w = std::max(write[(k + 2) % 3], o) + S * img / kPageableBytesUs;
+  }
+  return *std::max_element(write, write + 3);
+}
+
+// Chunks of the host calls: slices per chunk; chunks are multiples of unit.
 struct HostPlan {
-  int64_t C, unit;  // slices per chunk; chunks are multiples of unit
+  int64_t C, unit;
 };
-HostPlan host_plan(const ctas_fbp *h, int64_t S, bool wb, bool pinned) {
+
+// Groups of four need chunks of at least four slices, whose copies overlap less: four
+// slices of 180 x 4096, bound by their copies, took 6.7 ms in one chunk and 5.5 ms in
+// four.  The faster of both is taken, by the estimate us(plan).
+template <class F> HostPlan host_chunks(const ctas_fbp *h, int64_t S, bool wb, F us) {
   if (h->chunk > 0) return {std::min<int64_t>(h->chunk, S), 1};
   // a chunk's buffers in at most 1 GB: rows, filtered rows (and their dense copy where
   // groups are written back), slices
@@ -721,13 +749,25 @@ HostPlan host_plan(const ctas_fbp *h, int64_t S, bool wb, bool pinned) {
   int64_t cmax = std::max<int64_t>(1, (int64_t)(1.0e9 / per));
   // keep at least a few chunks so copies overlap compute
   cmax = std::min<int64_t>(cmax, std::max<int64_t>(1, (S + 3) / 4));
-  const int64_t nch = (S + cmax - 1) / cmax, C = (S + nch - 1) / nch, u = ctas::kQuadSlices;
-  const int64_t G = std::min(S, quad_groups(C) * u);
-  if (quad_count(h, G) == 0) return {C, 1};
-  if ((h->flags & CTAS_FLAG_GROUPS) ||
-      plan_us(h, chunk_plan(S, G, u), wb, pinned) < 0.97 * plan_us(h, chunk_plan(S, C, 1), wb, pinned))
-    return {G, u};
-  return {C, 1};
+  const int64_t nch = (S + cmax - 1) / cmax, u = ctas::kQuadSlices;
+  const HostPlan plain{(S + nch - 1) / nch, 1}, groups{std::min(S, quad_groups(plain.C) * u), u};
+  if (quad_count(h, groups.C) == 0) return plain;
+  return (h->flags & CTAS_FLAG_GROUPS) || us(groups) < 0.97 * us(plain) ? groups : plain;
+}
+
+HostPlan host_plan(const ctas_fbp *h, int64_t S, bool wb, bool pinned) {
+  return host_chunks(h, S, wb, [&](const HostPlan &p) {
+    return plan_us(h, chunk_plan(S, p.C, p.unit), wb, pinned);
+  });
+}
+
+// The volume call's chunks.  By the stack call's estimate, without the callbacks that
+// bound it, four slices of 1800 x 2560 went in one chunk: 33 ms, where four
+// chunks take 25 (callbacks of numpy copies; 16-bit samples 22 and 14 ms).
+int64_t volume_chunk(const ctas_fbp *h, int64_t S, int64_t sample_bytes) {
+  return host_chunks(h, S, false, [&](const HostPlan &p) {
+           return volume_us(h, S, p.C, sample_bytes);
+         }).C;
 }
 
 bool is_pinned(const void *p) {
@@ -1389,7 +1429,7 @@ int ctas_fbp_reconstruct_volume(ctas_fbp *h, int64_t n_slices, float center, int
     const bool own_range = bpp != 0 && mincon == maxcon;
     int64_t C = 0;
     StackBuffers sized(h, [&] {
-      C = host_plan(h, n_slices, false, true).C;  // through the pinned rings
+      C = volume_chunk(h, n_slices, sb);
       for (auto &w : h->ws) {
         ensure_set(h, w, C, true, h->stream);
         if (bpp != 0) w.samples.ensure((size_t)(sb * C * OO));
