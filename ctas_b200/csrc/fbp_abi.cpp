@@ -329,7 +329,10 @@ void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw, cudaStream_t 
     if (w.quad.ensure(sizeof(float) * ctas::kQuadSlices * (size_t)words))
       cuda_check(cudaMemsetAsync(w.quad.p, 0, w.quad.bytes, st), "cudaMemsetAsync");
   }
-  if (w.filt.ensure(elem_bytes(h->store) * (size_t)(alone * N * h->Wp)))
+  const size_t rows = elem_bytes(h->store) * (size_t)(alone * N * h->Wp);
+  // sino()'s rows go with the old buffer, also where the call fails after this
+  if (rows > w.filt.bytes) h->have_sino = false;
+  if (w.filt.ensure(rows))
     cuda_check(cudaMemsetAsync(w.filt.p, 0, w.filt.bytes, st), "cudaMemsetAsync");
   if (h->store != 0) w.scale.ensure(sizeof(float) * (size_t)(S * N));
   w.slice.ensure(sizeof(float) * (size_t)(S * h->out_rows * h->out_cols));
