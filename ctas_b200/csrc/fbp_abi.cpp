@@ -107,6 +107,30 @@ struct DevBuf {
   ~DevBuf() { release(); }
 };
 
+// Filtered rows: those of the one-slice kernel, and behind them the interleaved rows of
+// the four-slice groups, with their slack.  One allocation, since each takes 0.34 ms,
+// whatever its size: the first call of a handle with five slices of 901 x 1023 took
+// 1.82 ms in two, 1.49 in one.
+struct RowBuf {
+  DevBuf buf;
+  size_t alone = 0, quad = 0;  // bytes of each part
+  bool holds(size_t a, size_t q) const { return a <= alone && q <= quad; }
+  void grow(size_t a, size_t q) {
+    a = std::max(alone, (a + 255) / 256 * 256);
+    q = std::max(quad, q);
+    release();
+    buf.ensure(a + q);
+    alone = a;
+    quad = q;
+  }
+  void release() {
+    buf.release();
+    alone = quad = 0;
+  }
+  template <class T> T *filt() const { return buf.as<T>(); }
+  float *groups() const { return reinterpret_cast<float *>(buf.as<char>() + alone); }
+};
+
 // Device constants of one reconstruction set-up, shared by clones.
 struct Consts {
   int device = 0;
@@ -127,8 +151,8 @@ struct QuadNeed {
 
 // One set of work buffers (the host stack call double-buffers two sets).
 struct WorkSet {
-  DevBuf raw, filt, scale, slice, part, minmax, ring_avg, ring;
-  DevBuf quad;     // interleaved rows of the four-slice groups, with their slack
+  DevBuf raw, scale, slice, part, minmax, ring_avg, ring;
+  RowBuf rows;     // filtered rows
   DevBuf dense;    // dense filtered rows to be written back (four-slice groups)
   DevBuf samples;  // converted output samples of the volume call
   int64_t slices = 0;
@@ -199,7 +223,7 @@ struct ctas_fbp {
       if (w.ev_done) cudaEventDestroy(w.ev_done);
       if (w.ev_out) cudaEventDestroy(w.ev_out);
       w.raw.release();
-      w.filt.release();
+      w.rows.release();
       w.scale.release();
       w.slice.release();
       w.part.release();
@@ -207,7 +231,6 @@ struct ctas_fbp {
       w.ring_avg.release();
       w.ring.release();
       w.samples.release();
-      w.quad.release();
       w.dense.release();
     }
     for (auto *r : {vin, vout})
@@ -313,7 +336,7 @@ int64_t quad_resident(const ctas_fbp *h, int64_t groups) {
 
 // First row of the interleaved buffer.
 float *quad_rows(const WorkSet &w) {
-  return w.quad.as<float>() + ctas::kQuadSlices * ctas::kQuadSlack;
+  return w.rows.groups() + ctas::kQuadSlices * ctas::kQuadSlack;
 }
 
 // Sizes one work set for S slices or fewer.  The padded filtered buffers are zeroed
@@ -324,16 +347,15 @@ void ensure_set(ctas_fbp *h, WorkSet &w, int64_t S, bool need_raw, cudaStream_t 
   if (need_raw) w.raw.ensure(sizeof(float) * (size_t)(S * N * W));
   const QuadNeed need = quad_need(h, S);
   const int64_t alone = h->store == CTAS_STORE_F32 ? need.alone : S;
-  if (need.groups > 0) {
-    const int64_t words = quad_resident(h, need.groups) * N * h->Wp + 2 * ctas::kQuadSlack;
-    if (w.quad.ensure(sizeof(float) * ctas::kQuadSlices * (size_t)words))
-      cuda_check(cudaMemsetAsync(w.quad.p, 0, w.quad.bytes, st), "cudaMemsetAsync");
+  const size_t filt = elem_bytes(h->store) * (size_t)(alone * N * h->Wp);
+  const int64_t words =
+      need.groups > 0 ? quad_resident(h, need.groups) * N * h->Wp + 2 * ctas::kQuadSlack : 0;
+  const size_t quad = sizeof(float) * ctas::kQuadSlices * (size_t)words;
+  if (!w.rows.holds(filt, quad)) {
+    h->have_sino = false;  // sino()'s rows go with the old buffer, also where the call fails after this
+    w.rows.grow(filt, quad);
+    cuda_check(cudaMemsetAsync(w.rows.buf.p, 0, w.rows.buf.bytes, st), "cudaMemsetAsync");
   }
-  const size_t rows = elem_bytes(h->store) * (size_t)(alone * N * h->Wp);
-  // sino()'s rows go with the old buffer, also where the call fails after this
-  if (rows > w.filt.bytes) h->have_sino = false;
-  if (w.filt.ensure(rows))
-    cuda_check(cudaMemsetAsync(w.filt.p, 0, w.filt.bytes, st), "cudaMemsetAsync");
   if (h->store != 0) w.scale.ensure(sizeof(float) * (size_t)(S * N));
   w.slice.ensure(sizeof(float) * (size_t)(S * h->out_rows * h->out_cols));
   if (h->contrast == CTAS_ABS) {
@@ -358,7 +380,7 @@ struct StackBuffers {
     } catch (const ctas::Error &e) {
       if (e.code != CTAS_E_NOMEM || !quad_capable(h)) throw;
       for (auto &w : h->ws) {
-        w.quad.release();
+        w.rows.release();
         w.dense.release();
       }
       h->singles = true;
@@ -424,7 +446,8 @@ const float *run_ring(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaSt
 }
 
 // Filter S slices of x (device, dense S x N x W): with float32 rows the first
-// quad_count() into w.quad, all others into w.filt; densely into `dense` too, unless null (float32 store).
+// quad_count() into w.rows.groups(), all others into w.rows.filt(); densely into `dense`
+// too, unless null (float32 store).
 void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t st,
                 float *dense = nullptr) {
   const float *ring = run_ring(h, x, S, w, st);
@@ -437,7 +460,7 @@ void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t
   ctas::FilterLaunch a{};
   a.x = x;
   a.x_slice_stride = h->N * h->W;
-  a.q = w.filt.p;
+  a.q = w.rows.filt<void>();
   a.q_slice_stride = h->N * h->Wp;
   a.row_scale = h->store ? w.scale.as<float>() : nullptr;
   a.tw = h->dc->tw.as<float2>();
@@ -483,7 +506,7 @@ void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t
     cuda_check(ctas::launch_filter(a, st), "filter kernel");
     h->launches += 1;
     if (h->wide) {
-      cuda_check(ctas::launch_halo(w.filt.as<float>(), h->N * h->Wp, (int)h->N, (int)h->W,
+      cuda_check(ctas::launch_halo(w.rows.filt<float>(), h->N * h->Wp, (int)h->N, (int)h->W,
                                    (int)h->Wp, (int)h->off, (int)rest, st),
                  "halo kernel");
       h->launches += 1;
@@ -497,7 +520,7 @@ void run_filter(ctas_fbp *h, const float *x, int64_t S, WorkSet &w, cudaStream_t
 void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, cudaStream_t st,
             const float *centers_dev = nullptr) {
   ctas::BpLaunch b{};
-  b.q = w.filt.p;
+  b.q = w.rows.filt<void>();
   b.q_slice_stride = centers_dev ? 0 : h->N * h->Wp;
   b.centers = centers_dev;
   b.row_scale = h->store ? w.scale.as<float>() : nullptr;
@@ -536,7 +559,7 @@ void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, 
       g.S = (int)std::min(step, n4 - s0);
       g.out = out + s0 * b.out_slice_stride;
       if (h->store != CTAS_STORE_F32) {
-        cuda_check(ctas::launch_expand_quad(w.filt.as<char>() + elem_bytes(h->store) * s0 * h->N * h->Wp,
+        cuda_check(ctas::launch_expand_quad(w.rows.filt<char>() + elem_bytes(h->store) * s0 * h->N * h->Wp,
                                             h->N * h->Wp, w.scale.as<float>() + s0 * h->N, h->store,
                                             (int)h->N, (int)h->Wp, g.S, quad_rows(w), st),
                    "expansion kernel");
@@ -553,8 +576,8 @@ void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, 
     if (n4 == S) return;
     b.S = (int)(S - n4);
     b.out = out + n4 * b.out_slice_stride;
-    if (h->store != CTAS_STORE_F32) {  // all of the 16-bit rows are in w.filt
-      b.q = w.filt.as<char>() + elem_bytes(h->store) * n4 * h->N * h->Wp;
+    if (h->store != CTAS_STORE_F32) {  // all of the 16-bit rows are in w.rows.filt()
+      b.q = w.rows.filt<char>() + elem_bytes(h->store) * n4 * h->N * h->Wp;
       b.row_scale += n4 * h->N;
     }
   }
@@ -582,18 +605,18 @@ void run_bp(ctas_fbp *h, const WorkSet &w, int64_t S, float center, float *out, 
 }
 
 // Copies the filtered rows of w's first S slices to the host rows `dst`
-// (dense S x N x W) on `st`.  Float32 stores: one pitched copy from w.filt,
+// (dense S x N x W) on `st`.  Float32 stores: one pitched copy from w.rows.filt(),
 // W samples from column off of each Wp-sample row.  16-bit stores: the
 // stored samples times their row scales, formed by the unpad kernel in w.raw.
 void writeback_rows(ctas_fbp *h, WorkSet &w, int64_t S, float *dst, cudaStream_t st) {
   if (h->store == 0) {
-    cuda_check(cudaMemcpy2DAsync(dst, sizeof(float) * (size_t)h->W, w.filt.as<float>() + h->off,
+    cuda_check(cudaMemcpy2DAsync(dst, sizeof(float) * (size_t)h->W, w.rows.filt<float>() + h->off,
                                  sizeof(float) * (size_t)h->Wp, sizeof(float) * (size_t)h->W,
                                  (size_t)(S * h->N), cudaMemcpyDeviceToHost, st),
                "cudaMemcpy2DAsync");
     return;
   }
-  cuda_check(ctas::launch_unpad(w.filt.p, h->N * h->Wp, w.scale.as<float>(), h->store, (int)h->N,
+  cuda_check(ctas::launch_unpad(w.rows.filt<void>(), h->N * h->Wp, w.scale.as<float>(), h->store, (int)h->N,
                                 (int)h->W, (int)h->Wp, (int)S, w.raw.as<float>(), h->N * h->W, st,
                                 (int)h->off),
              "unpad kernel");
@@ -1207,7 +1230,7 @@ int ctas_fbp_sino_dev(ctas_fbp *h, const float *sino_dev, float *filtered_dev, v
     ensure_set(h, w, 1, false, st);
     run_filter(h, sino_dev, 1, w, st);
     if (filtered_dev) {
-      cuda_check(ctas::launch_unpad(w.filt.p, h->N * h->Wp, h->store ? w.scale.as<float>() : nullptr,
+      cuda_check(ctas::launch_unpad(w.rows.filt<void>(), h->N * h->Wp, h->store ? w.scale.as<float>() : nullptr,
                                     h->store, (int)h->N, (int)h->W, (int)h->Wp, 1, filtered_dev,
                                     h->N * h->W, st, (int)h->off),
                  "unpad kernel");
@@ -1375,7 +1398,7 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
       // 16-bit stores: the written-back rows are the stored samples times
       // their row scales, formed by the unpad kernel in w.raw
       if (wb && h->store != 0) {
-        cuda_check(ctas::launch_unpad(w.filt.p, h->N * h->Wp, w.scale.as<float>(), h->store,
+        cuda_check(ctas::launch_unpad(w.rows.filt<void>(), h->N * h->Wp, w.scale.as<float>(), h->store,
                                       (int)h->N, (int)h->W, (int)h->Wp, (int)S,
                                       w.raw.as<float>(), NW, h->stream, (int)h->off),
                    "unpad kernel");
@@ -1391,11 +1414,11 @@ int ctas_fbp_reconstruct_stack(ctas_fbp *h, float *sinos, float *slices, int64_t
                                    cudaMemcpyDeviceToHost, h->s_out),
                    "cudaMemcpyAsync");
       } else if (wb && h->store == 0) {
-        // float32 store: the filtered rows sit in w.filt, W samples from column
+        // float32 store: the filtered rows sit in w.rows.filt(), W samples from column
         // off of every Wp-sample row (slices follow at N rows each), and one
         // pitched copy brings them back
         cuda_check(cudaMemcpy2DAsync(sinos + s0 * NW, sizeof(float) * (size_t)h->W,
-                                     w.filt.as<float>() + h->off, sizeof(float) * (size_t)h->Wp,
+                                     w.rows.filt<float>() + h->off, sizeof(float) * (size_t)h->Wp,
                                      sizeof(float) * (size_t)h->W, (size_t)(S * h->N),
                                      cudaMemcpyDeviceToHost, h->s_out),
                    "cudaMemcpy2DAsync");
