@@ -394,10 +394,11 @@ __device__ __forceinline__ void filter_pair(const FilterLaunch &a, int pair, int
   // rows go straight from the last inverse stage to global memory unless a
   // row-wide epilogue (REF running sum, reduced-precision scale) needs them
   const bool direct = ns >= 2 && a.contrast != 1 && a.store == 0;
-  // es: elements between samples of a row, ep: between rows
+  // es: elements between samples of a row, ep: between rows (in 64 bits the plain form
+  // took 79.9 us for 1800 rows of 2560, in 32 78.6)
   const bool quad = GROUP && a.quad;
   const int es = quad ? kQuadSlices : 1;
-  const int64_t ep = (int64_t)es * a.Wp;
+  const int ep = es * a.Wp;
   T *q0 = reinterpret_cast<T *>(a.q) + (quad ? (sl / kQuadSlices) * a.q_slice_stride + sl % kQuadSlices
                                              : sl * a.q_slice_stride) +
           (int64_t)r0 * ep + (a.off ? a.off : kRowOff) * es;
