@@ -13,9 +13,9 @@
 // shortens the call (three_pays): the filter is bound by its passes over P elements in
 // shared memory (6144 instead of 8192 for rows of 2560).  The choice does not depend on
 // the number of images, so that a batch equals single calls.  5 2^k (5120 there) ran in
-// 0.94 ms where 3 2^k takes 1.16 ms on 31 x 1024 x 2560, but its rounding error on rows whose mean is small against their
-// range is up to 10 % above that of 2^k, in every form of the twiddles and the mean
-// (filter.cu), and is not used.
+// 0.94 ms where 3 2^k takes 1.11 ms on 31 x 1024 x 2560, but its rounding error on rows
+// whose mean is small against their range is up to 10 % above that of 2^k, in every form
+// of the twiddles and the mean (filter.cu), and is not used.
 //
 // Backprojection.  One thread per result pixel adds the n images' terms in
 // order, with the reference's float expression for the sample index.
@@ -174,8 +174,9 @@ std::vector<double> ts_window(const std::vector<float> &fwin, int64_t n, int64_t
 // Whether the transform of 3 2^k, which costs a pass for the rows' mean and longer
 // twiddle tables, is the faster one: where 2^k is 8192 or 16384 and the row pairs of one
 // image more than its CTAs that the device holds (three and one to an SM).  9 images of
-// 1024 x 1500 take 183 us at 4096 and 198 at 3072; one of 256 x 2560 39 us at 8192 and 42
-// at 6144, of 1024 x 2560 78 and 65, 31 of 1024 x 6000 5.8 and 3.6 ms.
+// 1024 x 1500 take 185 us at 4096 and 203 at 3072; one of 256 x 2560 42 us at 8192 and 41
+// at 6144, of 800 x 2560 61 and 57, of 1024 x 2560 81 and 67; one of 256 x 6000 63 us at
+// 16384 and 67 at 12288, 31 of 1024 x 6000 5.8 and 3.4 ms.
 bool three_pays(int64_t P, int64_t rows, int sms) {
   return P >= 8192 && (rows + 1) / 2 > (int64_t)sms * (P == 8192 ? 3 : 1);
 }
